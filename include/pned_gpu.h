@@ -198,6 +198,16 @@ int pned_tile_plan_export(const pned_model_desc *d, int row_bits, const pned_til
  */
 int pned_qtile_plan_export(const pned_model_desc *d, int k, int low, int64_t *out, int64_t cap, int64_t *len);
 /*
+ * Test hook (no counterpart in the reference): the passes of the class-tiled
+ * kernel (S = 1/2 full basis) for R vectors, computed on the host.  out[0..cap)
+ * receives int64 values, *len the full count: lr (groups of 2^lr vectors), the
+ * number of flip terms X, X records (xmask, pos4, tab, nb), the number of
+ * passes, and per pass (nrow, nouter, nmembers, nout, ntab), rowpos[nrow],
+ * jpos[3], outer[nouter], nmembers records (dmask, mul, mask, pack) -- the first
+ * nout out-of-tile -- and the source entry of each table entry (-1: unused).
+ */
+int pned_xtile_plan_export(const pned_model_desc *d, int R, int64_t *out, int64_t cap, int64_t *len);
+/*
  * Measurement hook (no counterpart in the reference): the partner-tile
  * staging the single-vector plan actually runs (0 gathered through L1/L2,
  * 1 cp.async, 2 bulk copies) and, for 2, the number of ring stages.

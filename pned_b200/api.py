@@ -447,6 +447,30 @@ def qtile_plan_export(desc: "ModelInput", k: int, low: int = 0) -> dict:
     return {"q": q, "n": nsites, "rterms": rterms, "nonzero": nonzero, "passes": passes}
 
 
+def xtile_plan_export(desc: "ModelInput", R: int) -> dict:
+    """The class-tiled passes (S = 1/2 full basis) for R vectors, computed on the
+    host (pned_xtile_plan_export)."""
+    n = C.c_int64(0)
+    check(lib().pned_xtile_plan_export(C.byref(desc.c), int(R), None, 0, C.byref(n)))
+    buf = np.zeros(n.value, dtype=np.int64)
+    check(lib().pned_xtile_plan_export(C.byref(desc.c), int(R), buf.ctypes.data_as(C.POINTER(C.c_int64)), n.value,
+                                       C.byref(n)))
+    it = iter(buf.tolist())
+    lr, nx = next(it), next(it)
+    xterms = [dict(zip(("xmask", "pos4", "tab", "nb"), (next(it) for _ in range(4)))) for _ in range(nx)]
+    passes = []
+    for _ in range(next(it)):
+        nrow, nouter, nsub, nout, ntab = (next(it) for _ in range(5))
+        ps = {"nout": nout}
+        ps["rowpos"] = [next(it) for _ in range(nrow)]
+        ps["jpos"] = [next(it) for _ in range(3)]
+        ps["outer"] = [next(it) for _ in range(nouter)]
+        ps["members"] = [dict(zip(("dmask", "mul", "mask", "pack"), (next(it) for _ in range(4)))) for _ in range(nsub)]
+        ps["tsrc"] = [next(it) for _ in range(ntab)]
+        passes.append(ps)
+    return {"lr": lr, "xterms": xterms, "passes": passes}
+
+
 class Model:
     """A compiled model on the current device (pned_model_create)."""
 

@@ -990,6 +990,8 @@ int64_t rtile_dynamic_partials(const pned_model *m, int R, int nblocks)
 bool tile_dynamic(const pned_model *m, const HvArgs &a, int nblocks)
 {
     if (!a.tile_counter) return false;
+    if (const pned_model::XTileSet *xs = find_xtiles(m, a.R))
+        return xtile_rows(m, *xs, a.R, nblocks, true) * a.K * a.R <= a.partials_cap;
     if (a.R == 1) {
         if (m->tprogs.empty() || !m->use_tile || tile_staged(m)) return false;
         return tile_dynamic_partials(m) * a.K <= a.partials_cap;
@@ -1000,6 +1002,8 @@ bool tile_dynamic(const pned_model *m, const HvArgs &a, int nblocks)
 
 int64_t hv_partials(const pned_model *m, const HvArgs &a, int nblocks)
 {
+    if (const pned_model::XTileSet *xs = find_xtiles(m, a.R))
+        return xtile_rows(m, *xs, a.R, nblocks, tile_dynamic(m, a, nblocks));
     if (tile_dynamic(m, a, nblocks))
         return a.R == 1 ? tile_dynamic_partials(m) : rtile_dynamic_partials(m, a.R, nblocks);
     return hv_partial_blocks(m, a.R, nblocks);
@@ -1007,6 +1011,7 @@ int64_t hv_partials(const pned_model *m, const HvArgs &a, int nblocks)
 
 int hv_partial_blocks(const pned_model *m, int R, int nblocks)
 {
+    if (const pned_model::XTileSet *xs = find_xtiles(m, R)) return int(xtile_rows(m, *xs, R, nblocks, false));
     if (!m->tprogs.empty() && R == 1 && m->use_tile) return int(m->tprogs.size()) * tile_grid(m, nblocks);
     if (const pned_model::TileSet *ts = find_rtiles(m, R)) return int(ts->progs.size()) * rtile_grid(m, nblocks);
     if (const pned_model::QTileSet *qs = find_qtiles(m, R)) return int(qs->progs.size()) * qtile_grid(m, *qs, nblocks);
@@ -1016,6 +1021,7 @@ int hv_partial_blocks(const pned_model *m, int R, int nblocks)
 
 cudaError_t launch_hv(const pned_model *m, const HvArgs &a, int nblocks, cudaStream_t st)
 {
+    if (const pned_model::XTileSet *xs = find_xtiles(m, a.R)) return launch_xtile(m, *xs, a, nblocks, st);
     if (!m->tprogs.empty() && a.R == 1 && m->use_tile) {
         if (tile_staged(m)) return launch_tile_staged(m, a, nblocks, st);
         if (m->tile_stage == 3 && tile_tma_usable(m, a)) return launch_tile_tma(m, a, nblocks, st);
@@ -1413,7 +1419,7 @@ extern "C" int pned_model_destroy(pned_model *m)
 extern "C" int pned_model_tile_staging(const pned_model *m, int *mode, int *ring_stages)
 {
     if (!m) return fail(PNED_EINVAL, "pned_model_tile_staging: null model");
-    const int md = m->use_tile ? m->tile_stage : 0;
+    const int md = m->use_tile && !find_xtiles(m, 1) ? m->tile_stage : 0;
     if (mode) *mode = md;
     if (ring_stages) *ring_stages = md == 2 ? m->bulk_stages : 0;
     return PNED_OK;
@@ -1431,7 +1437,11 @@ extern "C" int pned_model_plan(const pned_model *m, int R, int *tile_passes, int
 {
     if (!m || R < 1) return fail(PNED_EINVAL, "pned_model_plan: bad arguments");
     int passes = 0, groups = 0, states = 0;
-    if (R == 1 && m->use_tile) {
+    if (const pned_model::XTileSet *xs = find_xtiles(m, R)) {
+        passes = int(xs->progs.size());
+        groups = xs->groups;
+        states = kXTile >> xs->lr;
+    } else if (R == 1 && m->use_tile) {
         passes = int(m->tprogs.size());
         for (const auto &t : m->tprogs) groups += t->ngroups;
         states = kThreads * (1 << m->tile_jb);
@@ -1457,6 +1467,14 @@ extern "C" int pned_model_plan(const pned_model *m, int R, int *tile_passes, int
     return PNED_OK;
 }
 
+namespace pned {
+bool plan_default(const pned_tile_plan *p)
+{
+    return !p || (p->row_fixed_bits < 0 && p->window_bits < 0 && p->max_passes < 0 && p->j_bits < 0 &&
+                  p->stage_partner_tiles <= 0 && p->blocks_per_sm < 0 && p->objective < 0 && p->terms_in_flight < 0);
+}
+}  // namespace pned
+
 extern "C" int pned_model_set_plan(pned_model *m, int R, const pned_tile_plan *plan)
 {
     if (!m || pick_vpt(R) == 0) return fail(PNED_EINVAL, "pned_model_set_plan: bad arguments");
@@ -1468,10 +1486,19 @@ extern "C" int pned_model_set_plan(pned_model *m, int R, const pned_tile_plan *p
         m->plan1_set = plan != nullptr;
         m->carveout = m->plan1.l1_carveout != 0;
         build_tile_programs(m);
+        if (plan) clear_xtiles(m, 1);
+        else ensure_xtiles(m, 1, false);
         return PNED_OK;
     }
-    const pned_tile_plan def{-1, -1, -1, -1, -1, -1, -1, -1, -1};
     if (plan) m->carveout = plan->l1_carveout != 0;
+    if (plan_default(plan)) {   // the class-tiled passes, where they run
+        m->rtiles_set.erase(R);
+        if (ensure_xtiles(m, R, false)) return PNED_OK;
+    } else {
+        m->rtiles_set.insert(R);
+        clear_xtiles(m, R);
+    }
+    const pned_tile_plan def{-1, -1, -1, -1, -1, -1, -1, -1, -1};
     ensure_rtiles(m, R, false, plan ? plan : &def);
     return PNED_OK;
 }
@@ -1528,7 +1555,8 @@ extern "C" int pned_ctx_create(pned_model *m, int R, size_t budget, pned_ctx **o
     if (e != cudaSuccess) return cuda_fail(e, "cudaStreamCreate");
     c->stream = c->own_stream;
     // tiled kernels write one partial sum per block and pass
-    if (R > 1) ensure_rtiles(m, R, false, nullptr);
+    if (R == 1 ? !m->plan1_set : !m->rtiles_set.count(R)) ensure_xtiles(m, R, false);
+    if (R > 1 && !find_xtiles(m, R)) ensure_rtiles(m, R, false, nullptr);
     ensure_qtiles(m, R);
     // room for per-block sums, and for R = 1 for the per-tile sums of the dynamic tile
     // order: the current plan, or any plan of two passes with tiles of >= 2048 states
@@ -1541,10 +1569,12 @@ extern "C" int pned_ctx_create(pned_model *m, int R, size_t budget, pned_ctx **o
         pslots = std::max<size_t>(pslots, size_t(rtile_dynamic_partials(m, R, c->nblocks)) * kMaxK * R);
         pslots = std::max<size_t>(pslots, size_t(m->dim / 2048 + 1) * 2 * kMaxK * R);
     }
+    if (const pned_model::XTileSet *xs = find_xtiles(m, R))
+        pslots = std::max<size_t>(pslots, size_t(xtile_rows(m, *xs, R, c->nblocks, true)) * kMaxK * R);
     const size_t pbytes = sizeof(double2) * pslots;
     c->partials_cap = int64_t(pslots);
     e = cudaMalloc(&c->partials, pbytes);
-    if (e == cudaSuccess) e = cudaMalloc(&c->tile_ctr, sizeof(uint32_t) * kTileMaxPasses);
+    if (e == cudaSuccess) e = cudaMalloc(&c->tile_ctr, sizeof(uint32_t) * kTileCounters);
     if (e == cudaSuccess) e = cudaMalloc(&c->sums, sizeof(double2) * kMaxK * kMaxR * 4);
     if (e == cudaSuccess) e = cudaMalloc(&c->scal, sizeof(double) * kScalSlots * kMaxR);
     if (e == cudaSuccess) e = cudaMallocHost(&c->h_sums, sizeof(double2) * kMaxK * kMaxR * 4);

@@ -6,6 +6,7 @@
 #include <map>
 #include <memory>
 #include <mutex>
+#include <set>
 #include <vector>
 
 #include "kernels.cuh"
@@ -29,6 +30,14 @@ struct pned_model {
     };
     std::map<int, TileSet> rtiles;
     std::mutex rtiles_mu;
+    // class-tiled passes per R (q == 2, full basis; guarded by rtiles_mu): groups of 2^lr vectors
+    struct XTileSet {
+        std::vector<std::unique_ptr<pned::XTileProgram>> progs;
+        int lr = 0;
+        int groups = 0;   // partner tiles over all passes
+    };
+    std::map<int, XTileSet> xtiles;
+    std::set<int> rtiles_set;   // R > 1 with an explicit plan for the multi-vector kernel
     // tiled mixed-radix passes per R (q > 2, full basis; guarded by rtiles_mu)
     struct QTileSet {
         std::vector<std::unique_ptr<pned::QTileProgram>> progs;
@@ -110,7 +119,7 @@ struct pned_ctx {
     double2 *buf[pned::kMaxBuffers] = {nullptr, nullptr, nullptr, nullptr, nullptr, nullptr};
     double2 *partials = nullptr;   // [nblocks][kMaxK][kMaxR], or per-tile sums of the single-vector tile kernel
     int64_t partials_cap = 0;      // double2 slots at `partials`
-    uint32_t *tile_ctr = nullptr;  // [kTileMaxPasses] tile counters of the dynamic tile order
+    uint32_t *tile_ctr = nullptr;  // [kTileCounters] tile counters of the dynamic tile order
     double2 *sums = nullptr;       // [4][kMaxK*kMaxR]
     double *scal = nullptr;        // [kScalSlots][kMaxR]
     int *flag = nullptr;
@@ -125,6 +134,11 @@ __device__ __forceinline__ void cp_async16(void *smem_dst, const void *gmem_src)
 {
     const unsigned s = static_cast<unsigned>(__cvta_generic_to_shared(smem_dst));
     asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(s), "l"(gmem_src) : "memory");
+}
+__device__ __forceinline__ void cp_async8(void *smem_dst, const void *gmem_src)
+{
+    const unsigned s = static_cast<unsigned>(__cvta_generic_to_shared(smem_dst));
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 8;\n" ::"r"(s), "l"(gmem_src) : "memory");
 }
 __device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;\n" ::: "memory"); }
 template <int N> __device__ __forceinline__ void cp_async_wait()
@@ -163,6 +177,17 @@ void build_tile_programs(pned_model *m);
 bool ensure_rtiles(pned_model *m, int R, bool slot_tables, const pned_tile_plan *plan);
 // Shared memory of the tiled multi-vector kernel for R vectors.
 size_t rtile_smem(const pned_model *m, int R, bool slot_tables);
+// Class-tiled passes for R vectors (S = 1/2, n >= 12), once per model and R; false:
+// another kernel runs.  The set for R (null: none; clear_xtiles: an explicit plan takes
+// its place), the partial-sum rows a call writes, and all its passes.
+bool ensure_xtiles(pned_model *m, int R, bool slot_tables);
+const pned_model::XTileSet *find_xtiles(const pned_model *m, int R);
+void clear_xtiles(pned_model *m, int R);
+// No plan, or one whose every field asks for the default.
+bool plan_default(const pned_tile_plan *p);
+int64_t xtile_rows(const pned_model *m, const pned_model::XTileSet &xs, int R, int nblocks, bool dynamic);
+cudaError_t launch_xtile(const pned_model *m, const pned_model::XTileSet &xs, const HvArgs &a, int nblocks,
+                         cudaStream_t st);
 bool ensure_qtiles(pned_model *m, int R);
 // Tile set of the mixed-radix tiled kernel for R (null: the flat kernel runs).
 const pned_model::QTileSet *find_qtiles(const pned_model *m, int R);
@@ -276,6 +301,34 @@ __device__ __forceinline__ void tile_sums_store(double2 (&red)[K][1], double2 (*
         double2 sum = make_double2(0.0, 0.0);
         for (int w = 0; w < kThreads / 32; ++w) sum = cadd(sum, s_red[w][tid]);
         dst[tid] = sum;
+    }
+}
+
+constexpr int kXSPT = 1 << kXJB;             // states a thread of the class-tiled kernel
+constexpr int kXTile = kThreads * kXSPT;     // elements of its tiles
+constexpr int kXMaxVec = 8;                  // vectors of a tile of the class-tiled kernel
+// Block sums of the class-tiled kernel: lane r of each group of 2^lr holds vector r of the
+// block's group `ch`; dst[k][R] gets the group's columns.  The thread's sums are reset.
+template <int K>
+__device__ __forceinline__ void x_sums_store(double2 (&red)[K], double2 (*s_red)[K][kXMaxVec], int lr, int R, int ch,
+                                             double2 *dst)
+{
+    const uint32_t tid = threadIdx.x, rc = 1u << lr;
+#pragma unroll
+    for (int k = 0; k < K; ++k) {
+        for (uint32_t off = 16; off >= rc; off >>= 1) {
+            red[k].x += __shfl_xor_sync(0xffffffffu, red[k].x, off);
+            red[k].y += __shfl_xor_sync(0xffffffffu, red[k].y, off);
+        }
+        if ((tid & 31u) < rc) s_red[tid >> 5][k][tid & 31u] = red[k];
+        red[k] = make_double2(0.0, 0.0);
+    }
+    __syncthreads();
+    if (tid < uint32_t(K) * rc) {
+        const uint32_t k = tid >> lr, r = tid & (rc - 1u);
+        double2 sum = make_double2(0.0, 0.0);
+        for (int w = 0; w < kThreads / 32; ++w) sum = cadd(sum, s_red[w][k][r]);
+        dst[k * R + ch * rc + r] = sum;
     }
 }
 

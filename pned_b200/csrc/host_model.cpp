@@ -726,6 +726,305 @@ int plan_tiles(const HostProgram &P, int tbits, int jb, int fixed, int window_bi
     return PNED_OK;
 }
 
+// ---------------------------------------------------------------------------
+// Planner of the class-tiled kernel
+// ---------------------------------------------------------------------------
+namespace {
+
+// Tile bits (`size` of n, the `fixed` lowest among them) that hold the most
+// masks: greedy from every mask as the start, then exchanges of one bit while
+// more masks come inside; ties go to the set that touches more masks.
+uint32_t tile_most_masks(const std::vector<uint32_t> &masks, int n, int size, int fixed)
+{
+    const uint32_t low = (1u << fixed) - 1u;
+    auto score = [&](uint32_t t) {
+        int in = 0, touch = 0;
+        for (uint32_t m : masks) {
+            in += (m & ~t) == 0;
+            touch += (m & t) != 0;
+        }
+        return in * 4096 + touch;
+    };
+    uint32_t best = 0;
+    int bs = -1;
+    std::vector<uint32_t> starts{low};
+    for (uint32_t m : masks)
+        if (__builtin_popcount(low | m) <= size && std::find(starts.begin(), starts.end(), low | m) == starts.end())
+            starts.push_back(low | m);
+    for (uint32_t t : starts) {
+        while (__builtin_popcount(t) < size) {
+            int bb = -1, bv = -1;
+            for (int b = 0; b < n; ++b) {
+                if ((t >> b) & 1u) continue;
+                const int v = score(t | (1u << b));
+                if (v > bv) { bv = v; bb = b; }
+            }
+            t |= 1u << bb;
+        }
+        int v = score(t);
+        for (bool better = true; better;) {
+            better = false;
+            for (int a = fixed; a < n && !better; ++a) {
+                if (!((t >> a) & 1u)) continue;
+                for (int b = fixed; b < n; ++b) {
+                    if ((t >> b) & 1u) continue;
+                    const uint32_t t2 = (t & ~(1u << a)) | (1u << b);
+                    const int v2 = score(t2);
+                    if (v2 > v) { t = t2; v = v2; better = true; break; }
+                }
+            }
+        }
+        if (v > bs) { bs = v; best = t; }
+    }
+    return best;
+}
+
+// Variant of a term for J bits jp (see kXVarD): the smallest M that holds its J
+// dependencies under its J flips.
+int x_variant(const XorTerm &t, const int (&jp)[kXJB])
+{
+    int d = 0, m = 0;
+    for (int k = 0; k < kXJB; ++k) {
+        d |= int((t.xmask >> jp[k]) & 1u) << k;
+        for (int q = 0; q < t.nb; ++q)
+            if (int((t.pos4 >> (8 * q)) & 0xff) == jp[k]) m |= 1 << k;
+    }
+    int best = kXGeneric;
+    for (int v = 0; v < kXVariants; ++v)
+        if (kXVarD[v] == d && (m & ~kXVarM[v]) == 0 &&
+            (best == kXGeneric || __builtin_popcount(kXVarM[v]) < __builtin_popcount(kXVarM[best])))
+            best = v;
+    return best;
+}
+
+// Multiplier and width of a perfect hash of the values of `pos` bits (ascending):
+// (x * mul) >> (32 - width) differs for every x with bits among pos only.  Each bit
+// is moved to one of the top bits; where the moved copies collide for every order,
+// a wider hash is tried.  False: none found.
+bool bit_hash(const std::vector<int> &pos, uint32_t &mul, int &width)
+{
+    const int nd = int(pos.size());
+    if (nd == 0) { mul = 0; width = 0; return true; }
+    auto good = [&](uint32_t m, int w) {
+        uint64_t seen = 0;
+        for (int c = 0; c < (1 << nd); ++c) {
+            uint32_t x = 0;
+            for (int k = 0; k < nd; ++k) x |= uint32_t((c >> k) & 1) << pos[k];
+            const uint32_t h = (x * m) >> (32 - w);
+            if ((seen >> h) & 1u) return false;
+            seen |= uint64_t(1) << h;
+        }
+        return true;
+    };
+    for (int w = nd; w <= 6; ++w) {
+        std::vector<int> to;
+        for (int k = 0; k < w; ++k) to.push_back(32 - w + k);
+        do {   // pos[k] -> to[k]
+            uint32_t m = 0;
+            bool ok = true;
+            for (int k = 0; k < nd; ++k) {
+                if (to[k] < pos[k]) { ok = false; break; }
+                m |= 1u << (to[k] - pos[k]);
+            }
+            if (ok && good(m, w)) { mul = m; width = w; return true; }
+        } while (std::next_permutation(to.begin(), to.end()));
+    }
+    return false;
+}
+
+}  // namespace
+
+int plan_xtiles(const HostProgram &P, int sbits, int fixed, int max_passes, std::vector<XTilePass> &out)
+{
+    out.clear();
+    const int n = P.n;
+    if (P.q != 2 || P.sector || sbits < kXJB + 1 || fixed < 0 || fixed + kXJB > sbits || n <= sbits || n > 32 ||
+        max_passes < 1)
+        return PNED_ENOTSUP;
+    std::vector<uint32_t> tiles;
+    std::vector<std::vector<int>> take;   // terms of each pass
+    std::vector<int> left(P.xterms.size());
+    for (size_t i = 0; i < left.size(); ++i) left[i] = int(i);
+    while (int(tiles.size()) < max_passes && (tiles.empty() || !left.empty())) {
+        std::vector<uint32_t> masks;
+        for (int i : left) masks.push_back(P.xterms[i].xmask);
+        const uint32_t t = tile_most_masks(masks, n, sbits, fixed);
+        std::vector<int> in, rest;
+        for (int i : left) ((P.xterms[i].xmask & ~t) == 0 ? in : rest).push_back(i);
+        if (in.empty() && !tiles.empty()) break;
+        tiles.push_back(t);
+        take.push_back(in);
+        left = rest;
+    }
+    // masks outside every tile: the pass whose order gains the fewest outer bits
+    // (ties: the pass with fewer out-of-tile terms)
+    std::vector<uint32_t> win(tiles.size(), 0);
+    std::vector<int> nout(tiles.size(), 0);
+    while (!left.empty()) {
+        int bi = -1, bp = -1, bc = 1 << 20;
+        for (size_t k = 0; k < left.size(); ++k)
+            for (size_t p = 0; p < tiles.size(); ++p) {
+                const uint32_t m = P.xterms[left[k]].xmask;
+                const int c = __builtin_popcount(m & ~tiles[p] & ~win[p]) * 256 + nout[p];
+                if (c < bc) { bc = c; bi = int(k); bp = int(p); }
+            }
+        win[bp] |= P.xterms[left[bi]].xmask & ~tiles[bp];
+        ++nout[bp];
+        take[bp].push_back(left[bi]);
+        left.erase(left.begin() + bi);
+    }
+    for (size_t p = 0; p < tiles.size(); ++p) {
+        const uint32_t tile = tiles[p];
+        std::vector<uint32_t> masks;
+        for (int i : take[p]) masks.push_back(P.xterms[i].xmask);
+        std::vector<int> tb;
+        for (int b = 0; b < n; ++b)
+            if ((tile >> b) & 1u) tb.push_back(b);
+        // J bits: three tile bits above the fixed ones with the fewest classes (a member
+        // without a variant is a class of its own)
+        const int nt = int(tb.size());
+        uint32_t J = 0;
+        int bc = 1 << 20;
+        for (int a = fixed; a < nt; ++a)
+            for (int b = a + 1; b < nt; ++b)
+                for (int c = b + 1; c < nt; ++c) {
+                    const int jp[kXJB] = {tb[a], tb[b], tb[c]};
+                    const uint32_t j = (1u << jp[0]) | (1u << jp[1]) | (1u << jp[2]);
+                    std::vector<uint32_t> ks;
+                    int own = 0;
+                    for (int i : take[p]) {
+                        if (x_variant(P.xterms[i], jp) == kXGeneric) ++own;
+                        else ks.push_back(P.xterms[i].xmask & ~j);
+                    }
+                    std::sort(ks.begin(), ks.end());
+                    const int cl = own * 2 + int(std::unique(ks.begin(), ks.end()) - ks.begin());
+                    if (cl < bc) { bc = cl; J = j; }
+                }
+        XTilePass ps;
+        int nj = 0;
+        for (int b : tb) {
+            if ((J >> b) & 1u) ps.jpos[nj++] = b;
+            else ps.rowpos.push_back(b);
+        }
+        std::vector<std::pair<int, int>> ob;
+        for (int b = 0; b < n; ++b) {
+            if ((tile >> b) & 1u) continue;
+            int use = 0;
+            for (uint32_t m : masks) use += (m & ~tile) && ((m >> b) & 1u);
+            ob.push_back({-use, b});
+        }
+        std::sort(ob.begin(), ob.end());
+        for (auto &x : ob) ps.outer.push_back(x.second);
+        // classes in order of first appearance: out-of-tile ones by partner tile, then in-tile
+        struct Group { uint32_t key, part; bool in, own; std::vector<int> terms; };
+        std::vector<Group> groups;
+        for (int i : take[p]) {
+            const uint32_t m = P.xterms[i].xmask;
+            const uint32_t key = m & ~J;
+            auto it = std::find_if(groups.begin(), groups.end(), [&](const Group &g) { return g.key == key && !g.own; });
+            const bool own = x_variant(P.xterms[i], ps.jpos) == kXGeneric;
+            if (it == groups.end() || own) {
+                groups.push_back(Group{key, m & ~tile, (m & ~tile) == 0, own, {}});
+                it = groups.end() - 1;
+            }
+            it->terms.push_back(i);
+        }
+        std::stable_sort(groups.begin(), groups.end(), [](const Group &a, const Group &b) {
+            if (a.in != b.in) return !a.in;
+            return a.part < b.part;
+        });
+        for (size_t k = 0; k < groups.size(); ++k)
+            ps.groups += !groups[k].in && (k == 0 || groups[k].part != groups[k - 1].part);
+        auto jbits = [&](uint32_t m) {   // J bits of a mask
+            int d = 0;
+            for (int k = 0; k < kXJB; ++k) d |= int((m >> ps.jpos[k]) & 1u) << k;
+            return d;
+        };
+        for (const Group &g : groups) {
+            uint32_t cmask = g.key;
+            if (g.in) {
+                cmask = 0;
+                for (size_t k = 0; k < ps.rowpos.size(); ++k) cmask |= ((g.key >> ps.rowpos[k]) & 1u) << k;
+            }
+            bool first = true;
+            for (int i : g.terms) {
+                const XorTerm &t = P.xterms[i];
+                const int d = jbits(t.xmask), var = x_variant(t, ps.jpos);
+                // dependencies outside J (bit position, table index bit) and in J
+                std::vector<std::pair<int, int>> dep;
+                int jbit[kXJB] = {-1, -1, -1};
+                for (int k = 0; k < t.nb; ++k) {
+                    const int pos = (t.pos4 >> (8 * k)) & 0xff;
+                    bool inj = false;
+                    for (int q = 0; q < kXJB; ++q)
+                        if (ps.jpos[q] == pos) { jbit[q] = k; inj = true; }
+                    if (!inj) dep.push_back({pos, k});
+                }
+                std::sort(dep.begin(), dep.end());
+                std::vector<int> pos;
+                for (auto &x : dep) pos.push_back(x.first);
+                uint32_t mul = 0;
+                int width = 0;
+                if (!bit_hash(pos, mul, width)) return PNED_ENOTSUP;
+                XSub s{};
+                for (int q : pos) s.dmask |= 1u << q;
+                s.mul = mul;
+                s.mask = cmask;
+                const size_t tab = ps.tsrc.size();
+                if (tab > 0xffff) return PNED_ENOTSUP;
+                const int M = var == kXGeneric ? 7 : kXVarM[var], nj = __builtin_popcount(unsigned(M));
+                ps.tsrc.resize(tab + (size_t(1) << (width + nj)), -1);
+                for (int c = 0; c < (1 << int(pos.size())); ++c) {
+                    uint32_t x = 0;
+                    int idx = 0;
+                    for (size_t k = 0; k < pos.size(); ++k)
+                        if ((c >> k) & 1) { x |= 1u << pos[k]; idx |= 1 << dep[k].second; }
+                    const uint32_t h = width ? (x * mul) >> (32 - width) : 0u;
+                    for (int u = 0; u < (1 << nj); ++u) {
+                        int id = idx, i2 = 0;
+                        for (int k = 0; k < kXJB; ++k) {
+                            if (!((M >> k) & 1)) continue;
+                            if (((u >> i2) & 1) && jbit[k] >= 0) id |= 1 << jbit[k];
+                            ++i2;
+                        }
+                        ps.tsrc[tab + (size_t(h) << nj) + u] = t.tab + id;
+                    }
+                }
+                s.pack = uint32_t(var + 16 * d + (first ? 128 : 0)) | uint32_t(width ? 32 - width : 0) << 8 |
+                         uint32_t(tab) << 16;
+                first = false;
+                if (!g.in) ++ps.nout;
+                ps.subs.push_back(s);
+            }
+        }
+        if (ps.tsrc.size() > size_t(kXMaxTab)) return PNED_ENOTSUP;
+        out.push_back(ps);
+    }
+    return PNED_OK;
+}
+
+int plan_xtiles_for(const HostProgram &P, int R, int &lr, std::vector<XTilePass> &out)
+{
+    out.clear();
+    lr = 0;
+    // R = 3: groups of one vector would read 16 of every 48 bytes; the multi-vector kernel runs
+    // below 2^18 elements there are fewer tiles than resident blocks and a call is launch-bound:
+    // the other kernels are as fast (N = 14, R = 16: 0.116 ms both)
+    if (P.q != 2 || P.sector || P.n < 12 || R == 3 || double(P.dim) * R < double(1 << 18)) return PNED_ENOTSUP;
+    // Tiles of 2048 elements: up to 8 vectors of 2^(11 - lr) states.  A warp's global read
+    // moves 128 bytes a wavefront only from whole lines, so groups are as wide as R divides
+    // (8 vectors: 128-byte runs; N = 24, R = 16: 14.8 ms against 16.6 ms with groups of 4 and
+    // 25 ms with groups of 2), and narrower ones keep the low site bits in the tile (one
+    // vector: 4, N = 26: 3.74 ms against 3.85 with 3 and 3.78 with 5).
+    while (lr < 3 && R % (2 << lr) == 0) ++lr;
+    const int fixed[4] = {4, 2, 1, 0};
+    // Up to 2^22 elements (64 MB) the vectors stay in L2: one pass (N = 18, R = 16: 0.22 ms
+    // against 0.26 ms).  Beyond, two: their tiles hold most masks, so fewer partner tiles
+    // come from memory (N = 26, R = 4: 14.3 ms against 22.3 ms with one and 15.1 ms with three).
+    const int passes = double(P.dim) * R <= double(1 << 22) ? 1 : 2;
+    return plan_xtiles(P, 11 - lr, fixed[lr], passes, out);
+}
+
 }  // namespace pned
 
 // ---------------------------------------------------------------------------
@@ -881,6 +1180,38 @@ extern "C" int pned_tile_plan_export(const pned_model_desc *d, int row_bits, con
                                int64_t(t.hasj), int64_t(t.lmask)});
         for (int g = 0; g <= ng; ++g) v.push_back(ps.gstart[g]);
         for (int g = 0; g < ng; ++g) v.push_back(int64_t(ps.gxor[g]));
+    }
+    *len = int64_t(v.size());
+    for (int64_t i = 0; i < std::min<int64_t>(cap, *len); ++i) out[i] = v[size_t(i)];
+    return PNED_OK;
+}
+
+// Class-tiled passes of a model for R vectors as the kernel receives them, computed on
+// the host: the program's flip terms, then per pass the tile's bits, the members and
+// the table's source entries.
+extern "C" int pned_xtile_plan_export(const pned_model_desc *d, int R, int64_t *out, int64_t cap, int64_t *len)
+{
+    using namespace pned;
+    if (!d || !len || (cap > 0 && !out) || R < 1) return fail(PNED_EINVAL, "pned_xtile_plan_export: bad arguments");
+    HostProgram P;
+    int rc = compile_program(d, P);
+    if (rc) return rc;
+    int lr = 0;
+    std::vector<XTilePass> passes;
+    rc = plan_xtiles_for(P, R, lr, passes);
+    if (rc) return fail(rc, "pned_xtile_plan_export: no class-tiled plan for this model and R");
+    std::vector<int64_t> v{int64_t(lr), int64_t(P.xterms.size())};
+    for (const XorTerm &t : P.xterms) v.insert(v.end(), {int64_t(t.xmask), int64_t(t.pos4), int64_t(t.tab), int64_t(t.nb)});
+    v.push_back(int64_t(passes.size()));
+    for (const XTilePass &ps : passes) {
+        v.insert(v.end(), {int64_t(ps.rowpos.size()), int64_t(ps.outer.size()), int64_t(ps.subs.size()),
+                           int64_t(ps.nout), int64_t(ps.tsrc.size())});
+        for (int x : ps.rowpos) v.push_back(x);
+        for (int x : ps.jpos) v.push_back(x);
+        for (int x : ps.outer) v.push_back(x);
+        for (const XSub &q : ps.subs)
+            v.insert(v.end(), {int64_t(q.dmask), int64_t(q.mul), int64_t(q.mask), int64_t(q.pack)});
+        for (int x : ps.tsrc) v.push_back(x);
     }
     *len = int64_t(v.size());
     for (int64_t i = 0; i < std::min<int64_t>(cap, *len); ++i) out[i] = v[size_t(i)];

@@ -17,6 +17,7 @@ constexpr int kThreads = 256;
 constexpr int kMaxR = 16;
 constexpr int kMaxK = 4;          // reduction quantities per vector in one pass
 constexpr int kMaxVPT = 4;
+constexpr int kTileCounters = kTileMaxPasses * kMaxR;   // tile counters of the dynamic tile order
 
 struct __align__(16) dcplx { double x, y; };
 
@@ -75,6 +76,19 @@ struct TileProgram {
     uint16_t gstart[kTileMaxGroups + 1];
     uint32_t gxor[kTileMaxGroups];
     TileTerm t[kMaxTerms];
+};
+
+// One pass of the class-tiled kernel (see XSub): tiles of 256 * 8 elements --
+// `rc` = 2^lr of the R vectors times 2^(11 - lr) states.
+struct XTileProgram {
+    int lr, rbits;                    // row bits: 8 - lr
+    int nsub, nout, ntab, nouter;
+    int first, last, pass;
+    uint32_t jexp[1 << kXJB];         // global bits of the thread's j-th state
+    uint8_t rowpos[8];
+    uint8_t outer[32];
+    uint16_t tsrc[kXMaxTab];          // table entry -> entry of the model's table (0xffff: zero)
+    uint4 s[kMaxTerms + 1];           // members (XSub), one more read ahead
 };
 
 // Tensor-copy geometry of a single-vector tile (a pass's rows and j bits, in

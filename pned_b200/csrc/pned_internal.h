@@ -75,6 +75,41 @@ constexpr int kTileBigSites = 26;     // from here on the single-vector plan def
 constexpr int kTileMaxPasses = 4;
 constexpr int kTileMaxGroups = 64;    // partner tiles per pass
 
+// Class-tiled S = 1/2 program (the kernel of hv_xtile.cu).  A thread owns the
+// 2^3 states of three "J" bits; flip masks that differ only in J bits need the
+// same partner rows, so they form one class: the rows are loaded once and every
+// member (XSub) adds c(s) times them, its J part a fixed register permutation.
+//
+// One member: its coefficient depends on up to four state bits.  Those outside J
+// come from the thread's base as (base & dmask) * mul >> sh (a perfect hash found
+// by the planner), those in J (the set M) from the state; the pass's table holds
+// the values as tab + (hash << |M|) + (J bits of M, packed).  16 bytes, one
+// constant-bank read.
+struct XSub {
+    uint32_t dmask, mul;
+    uint32_t mask;     // the class's partner rows -- in-tile: local row xor; out-of-tile: global xor (no J bits)
+    uint32_t pack;     // variant + 16 * (J bits flipped) + 128 * (first of its class) + sh << 8 + tab << 16
+};
+// Variants, each with fixed J bits flipped (D) and fixed J dependencies (M): the ones
+// that two-site flips on lattices with few common neighbours need.  Any other member is
+// its own class under kXGeneric, its rows loaded with D applied and its table holding
+// all 8 J states per hash value.
+constexpr int kXVariants = 14, kXGeneric = 14;
+constexpr uint8_t kXVarD[kXVariants] = {0, 0, 0, 0, 0, 0, 0, 0, 1, 2, 4, 3, 5, 6};
+constexpr uint8_t kXVarM[kXVariants] = {0, 1, 2, 4, 3, 5, 6, 7, 1, 2, 4, 3, 5, 6};
+constexpr int kXJB = 3;         // J bits of a thread
+constexpr int kXMaxTab = 3072;  // table entries of a pass
+
+struct XTilePass {
+    std::vector<int> rowpos;   // global bits of the row bits, ascending
+    int jpos[kXJB] = {};       // global bits of the J bits
+    std::vector<int> outer;    // outer bits, fastest first
+    int nout = 0;              // members of out-of-tile classes come first
+    int groups = 0;            // distinct partner tiles
+    std::vector<XSub> subs;
+    std::vector<int> tsrc;     // table entry -> entry of the program's table (-1: unused)
+};
+
 struct QTilePass {
     std::vector<int> sites;              // tile sites, ascending: local digit k is site sites[k]
     std::vector<int> outer;              // the other sites, ascending
@@ -132,6 +167,14 @@ struct HostProgram {
 int plan_qtiles(const HostProgram &P, int k, int low, std::vector<QTilePass> &passes);
 int plan_tiles(const HostProgram &P, int tbits, int jb, int fixed, int window_bits, int max_passes,
                std::vector<HostProgram::TilePass> &out, int objective = 0);
+
+// Passes of the class-tiled kernel (q == 2, full basis, n > sbits): tiles of
+// sbits site bits, the `fixed` lowest among them.  Each pass's tile is chosen to
+// hold the most masks that are left; masks that no tile holds join the pass
+// whose tile order needs the fewest further bits for them.
+int plan_xtiles(const HostProgram &P, int sbits, int fixed, int max_passes, std::vector<XTilePass> &out);
+// The same with the tile shape and passes chosen for R vectors: groups of 2^lr of them.
+int plan_xtiles_for(const HostProgram &P, int R, int &lr, std::vector<XTilePass> &out);
 
 // Coefficient tables and diagonal tables of `d` evaluated on the term
 // structure of S (same lattice and bonds; q == 2): table[i] for the entries of

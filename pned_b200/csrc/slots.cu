@@ -618,8 +618,10 @@ extern "C" int pned_slots_create(const pned_model_desc *structure, int R, int ma
     // dynamic order (any plan of two passes with tiles of >= 2048 states)
     S->partials_cap = int64_t(S->nblocks) * kTileMaxPasses * kMaxK * kMaxR;
     if (R == 1) S->partials_cap = std::max<int64_t>(S->partials_cap, (S->dim / 2048 + 1) * 2 * kMaxK);
+    // and the per-chunk sums of the class-tiled kernel (tiles of 2048 elements, two passes)
+    S->partials_cap = std::max<int64_t>(S->partials_cap, (S->dim * R / 2048 + 1) * 2 * kMaxK * R / std::min(R, kXMaxVec));
     if (e == cudaSuccess) e = salloc(S.get(), &S->partials, size_t(S->partials_cap));
-    if (e == cudaSuccess) e = cudaMalloc(&S->tile_ctr, sizeof(uint32_t) * kTileMaxPasses);
+    if (e == cudaSuccess) e = cudaMalloc(&S->tile_ctr, sizeof(uint32_t) * kTileCounters);
     if (e == cudaSuccess) e = salloc(S.get(), &S->sums, size_t(12) * kMaxR);
     if (e == cudaSuccess) e = salloc(S.get(), &S->scratch, size_t(R) * 64 + size_t(R) * S->nbond * 4);
     if (e == cudaSuccess) e = cudaMemcpy(S->s1, hp.dsite1.data(), sizeof(int) * S->nbond, cudaMemcpyHostToDevice);
@@ -648,9 +650,9 @@ extern "C" int pned_slots_create(const pned_model_desc *structure, int R, int ma
         m.d_table = S->table; m.d_diag = S->diag;
         if (R == 1) {
             build_tile_programs(&m);
-            S->tile = m.use_tile;
+            S->tile = ensure_xtiles(&m, 1, false) || m.use_tile;
         } else {
-            S->tile = ensure_rtiles(&m, R, true, nullptr);
+            S->tile = ensure_xtiles(&m, R, true) || ensure_rtiles(&m, R, true, nullptr);
         }
     }
     *out = S.release();
@@ -854,9 +856,16 @@ extern "C" int pned_slots_set_plan(pned_slots *S, const pned_tile_plan *plan)
         S->tm.plan1_set = plan != nullptr;
         build_tile_programs(&S->tm);
         S->tile = S->tm.use_tile;
-    } else {
-        S->tile = ensure_rtiles(&S->tm, S->R, true, plan ? plan : &def);
     }
+    if (plan_default(plan)) {
+        if (ensure_xtiles(&S->tm, S->R, S->R > 1)) {
+            S->tile = true;
+            return PNED_OK;
+        }
+    } else {
+        clear_xtiles(&S->tm, S->R);
+    }
+    if (S->R > 1) S->tile = ensure_rtiles(&S->tm, S->R, true, plan ? plan : &def);
     return PNED_OK;
 }
 

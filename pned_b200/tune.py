@@ -47,7 +47,15 @@ CANDIDATES_R = [(-1, -1, -1), (0, 6, 2), (0, 8, 2), (0, 10, 2), (1, 10, 2), (3, 
                 (0, 6, 2, -1, 1, 0, -1, 1), (0, 8, 2, -1, 1, 0, -1, 1), (0, 10, 2, -1, 1, 0, -1, 1),
                 (1, 8, 2, -1, 1, 0, -1, 1), (0, 8, 3, -1, 1, 0, -1, 1), (0, 12, 1, -1, 1, 0, -1, 1)]
 
+# the library's own default: from 2^18 states on, complex couplings run the class-tiled kernel
+DEFAULT = (-1, -1, -1, -1)
+DEFAULT_DIM = 1 << 18
+
 _cache: dict = {}
+
+
+def _candidates_1(dim):
+    return [DEFAULT] + CANDIDATES_1 if dim >= DEFAULT_DIM else CANDIDATES_1
 
 
 def _device_name():
@@ -88,7 +96,7 @@ def autotune(model, R: int = 1, reps: int = 2, candidates=None, cache_path: str 
         best = _cache[key]
         model.set_plan(R, *best["plan"])
         return dict(best, cached=True)
-    cands = candidates or (CANDIDATES_1 if R == 1 else CANDIDATES_R)
+    cands = candidates or (_candidates_1(model.dim) if R == 1 else CANDIDATES_R)
     ctx = api.Context(model, R=R)
     v1 = torch.randn(model.dim * R, dtype=torch.complex128, device="cuda")
     v0 = torch.zeros_like(v1)
@@ -130,7 +138,7 @@ def autotune_slots(batch, structure, reps: int = 3, candidates=None) -> dict:
         return dict(_cache[key], cached=True)
     if batch.plan()["tile_passes"] == 0:
         return {"plan": [-1, -1, -1], "ms": None, "tried": []}
-    cands = candidates or (CANDIDATES_1 if batch.R == 1 else CANDIDATES_R)
+    cands = candidates or (_candidates_1(batch.dim) if batch.R == 1 else CANDIDATES_R)
     need = (reps + 1) * len(cands) + 2
     if need > batch.max_steps:
         cands = cands[:max(1, batch.max_steps // (reps + 1) - 1)]

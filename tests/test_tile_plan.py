@@ -317,3 +317,65 @@ def test_default_plan_below_26_sites_is_the_gather_plan():
     X, skip, pt = P.build_xlocal(2, 0, CP.kitaev_heisenberg(0.6, 1.6))
     d = P.ModelInput(cl.n, 2, 0, cl.ipair, cl.ibond_type, X, skip, pt)
     assert api.tile_plan_export(d) == api.tile_plan_export(d, 8, 10, -1, 3, objective=0)
+
+
+XTILE_CASES = [(14, 16, True), (16, 4, False), (18, 2, True), (18, 1, True), (18, 4, True), (18, 6, False), (20, 8, True),
+               (22, 1, True), (24, 12, False), (24, 16, True)]
+
+
+@pytest.mark.parametrize("n,R,field", XTILE_CASES)
+def test_class_tiled_plan_matches_every_flip_term(n, R, field):
+    """The class-tiled passes name every (state, flip term) pair exactly once: the
+    partner state and the coefficient-table entry of each member, followed through
+    the tile's rows, J bits, outer bits, hash and table as the kernel does, are the
+    ones of the flip term itself (sampled states, the lowest and the highest
+    included)."""
+    from pned_b200.lattice import cluster_for_sites
+    cl = cluster_for_sites(n)
+    cpl = CP.kitaev_heisenberg(0.6, 1.6, gamma=0.1 if field else 0.0)
+    X, skip, pt = P.build_xlocal(2, 0, cpl, field=CP.field_111(0.05) if field else None)
+    r = api.xtile_plan_export(P.ModelInput(n, 2, 0, cl.ipair, cl.ibond_type, X, skip, pt), R)
+    lr, D, M = r["lr"], [0, 0, 0, 0, 0, 0, 0, 0, 1, 2, 4, 3, 5, 6], [0, 1, 2, 4, 3, 5, 6, 7, 1, 2, 4, 3, 5, 6]
+    assert R % (1 << lr) == 0
+    dim = 1 << n
+    rng = np.random.default_rng(n + R)
+    s = np.unique(np.concatenate([[0, dim - 1], rng.integers(0, dim, 2000)])).astype(np.uint64)
+    tabsize = max(t["tab"] + (1 << t["nb"]) for t in r["xterms"])
+    want = set()
+    for t in r["xterms"]:
+        idx = np.zeros_like(s)
+        for k in range(t["nb"]):
+            idx |= ((s >> np.uint64((t["pos4"] >> (8 * k)) & 0xff)) & np.uint64(1)) << np.uint64(k)
+        want.add((tuple((s ^ np.uint64(t["xmask"])).tolist()), tuple((idx + np.uint64(t["tab"])).tolist())))
+    got = []
+    for ps in r["passes"]:
+        rows, jp = ps["rowpos"], ps["jpos"]
+        assert len(rows) + lr == 8 and sorted(rows + jp + ps["outer"]) == list(range(n))
+        jmask = np.uint64(sum(1 << b for b in jp))
+        base = s & ~jmask
+        j = sum((((s >> np.uint64(b)) & np.uint64(1)) << np.uint64(k)) for k, b in enumerate(jp))
+        new = False
+        for i, m in enumerate(ps["members"]):
+            var, flip, first = m["pack"] & 15, (m["pack"] >> 4) & 7, (m["pack"] >> 7) & 1
+            sh, tab = (m["pack"] >> 8) & 31, m["pack"] >> 16
+            new = new or first
+            assert new and (var < 14 or first)
+            # a variant flips its own J bits; the generic one has its rows loaded with the flip
+            assert var == 14 or D[var] == flip
+            mask = m["mask"]
+            if i >= ps["nout"]:   # local row xor
+                mask = sum(1 << b for k, b in enumerate(rows) if (m["mask"] >> k) & 1)
+                assert m["mask"] >> len(rows) == 0
+            assert mask & int(jmask) == 0
+            part = s ^ np.uint64(mask | sum(1 << b for k, b in enumerate(jp) if (flip >> k) & 1))
+            h = (((base & np.uint64(m["dmask"])) * np.uint64(m["mul"])) & np.uint64(0xffffffff)) >> np.uint64(sh)
+            mm = 7 if var == 14 else M[var]
+            u, nb = np.zeros_like(s), 0
+            for k in range(3):
+                if (mm >> k) & 1:
+                    u |= ((j >> np.uint64(k)) & np.uint64(1)) << np.uint64(nb)
+                    nb += 1
+            src = np.array(ps["tsrc"])[((h << np.uint64(nb)) + u + np.uint64(tab)).astype(np.int64)]
+            assert src.min() >= 0 and src.max() < tabsize
+            got.append((tuple(part.tolist()), tuple(src.tolist())))
+    assert len(got) == len(r["xterms"]) and set(got) == want
