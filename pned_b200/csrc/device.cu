@@ -152,6 +152,7 @@ __global__ void __launch_bounds__(kThreads) hv_xor_kernel(const __grid_constant_
         hv_epilogue<K, VPT>(a, s, r0, v, acc, scr, pcr, gsr, red);
     }
     block_reduce_store<K, VPT>(red, G, VPT, R, a.partials);
+    hv_finish(a);
 }
 
 // Tiled single-vector (R = 1) H.v on the S = 1/2 full basis, one pass of a
@@ -343,6 +344,7 @@ __global__ void __launch_bounds__(kThreads, BPS)
     }
     // static order: the block's sums over its tiles (same reduction order)
     if (!ctr) tile_sums_store<K>(red, s_red, a.partials + size_t(blockIdx.x) * K);
+    if (prog.last) hv_finish(a);
 }
 
 // Tiled multi-vector H.V (R > 1 interleaved vectors, S = 1/2 full basis), one
@@ -543,6 +545,7 @@ __global__ void __launch_bounds__(kThreads, 2) hv_tile_rv_kernel(const __grid_co
         chunk = s_next;
     }
     if (!ctr) block_reduce_store<K, VPT, true>(red, G, VPT, R, a.partials);
+    if (prog.last) hv_finish(a);
 }
 
 // Mixed-radix (q > 2) variant: partner = s + offset, coefficient indexed by
@@ -613,6 +616,7 @@ __global__ void __launch_bounds__(kThreads) hv_radix_kernel(const __grid_constan
         hv_epilogue<K, VPT>(a, s, r0, v, acc, scr, pcr, gsr, red);
     }
     block_reduce_store<K, VPT>(red, G, VPT, R, a.partials);
+    hv_finish(a);
 }
 
 // Sums partials[nb][KR] in a fixed order into out[KR] (one block).
@@ -663,11 +667,15 @@ __global__ void __launch_bounds__(kThreads) dot_kernel(const double2 *__restrict
     block_reduce_store<1, kMaxVPT>(red, G, vpt, R, partials);
 }
 
-// Lanczos residual: Rn = W - Re(alpha) v, beta^2 partial = sum |W - alpha v|^2 (v = sc C).
+// Lanczos residual: Rn = W - Re(alpha) v, beta^2 = sum |W - alpha v|^2 (v = sc C).  The
+// last block adds the blocks' sums and closes the step (the reference's S1/2
+// Lanczos.f90:111-130): alpha, beta recorded, the next scales set.  Two launches fewer a
+// step; N = 18 (everything in L2) is launch-bound.
 __global__ void __launch_bounds__(kThreads) residual_kernel(const double2 *__restrict__ W, const double2 *__restrict__ C,
                                                             double2 *Rn, const double *__restrict__ sc,
                                                             const double2 *__restrict__ alpha, int64_t dim, int R,
-                                                            int vpt, double2 *partials)
+                                                            int vpt, double2 *partials, const Finish fin,
+                                                            const LanczosTail tail)
 {
     double2 red[1][kMaxVPT];
     for (int j = 0; j < kMaxVPT; ++j) red[0][j] = make_double2(0.0, 0.0);
@@ -687,6 +695,20 @@ __global__ void __launch_bounds__(kThreads) residual_kernel(const double2 *__res
         }
     }
     block_reduce_store<1, kMaxVPT>(red, G, vpt, R, partials);
+    __shared__ double2 s_fin[kThreads];
+    if (!finish_last(fin, s_fin)) return;
+    const int k = *tail.counter, r = int(threadIdx.x);
+    __syncthreads();
+    if (r < R) {
+        const double be = sqrt(fin.out[r].x);
+        tail.alpha[(size_t)k * R + r] = alpha[r].x;
+        tail.beta[(size_t)k * R + r] = be;
+        if (!(be >= 0.5e-30)) atomicOr(tail.flag, 1);
+        const double old = tail.sc[r];
+        tail.sc[r] = 1.0 / be;
+        tail.pc[r] = -be * old;
+    }
+    if (r == 0) *tail.counter = k + 1;
 }
 
 
@@ -796,7 +818,8 @@ static cudaError_t launch_tile_j(const pned_model *m, const HvArgs &a, int nbloc
     const bool dyn = tile_dynamic(m, a, nblocks);
     HvArgs b = a;
     if (!dyn) b.tile_counter = nullptr;
-    else if ((e = cudaMemsetAsync(a.tile_counter, 0, sizeof(uint32_t) * kTileMaxPasses, st)) != cudaSuccess)
+    else if (!a.fin.out &&
+             (e = cudaMemsetAsync(a.tile_counter, 0, sizeof(uint32_t) * kTileMaxPasses, st)) != cudaSuccess)
         return e;
     size_t off = 0;
     for (size_t p = 0; p < m->tprogs.size(); ++p) {
@@ -937,7 +960,8 @@ static cudaError_t launch_rv_t(const pned_model *m, const pned_model::TileSet &t
     const bool dyn = tile_dynamic(m, a, nblocks);
     HvArgs b = a;
     if (!dyn) b.tile_counter = nullptr;
-    else if ((e = cudaMemsetAsync(a.tile_counter, 0, sizeof(uint32_t) * kTileMaxPasses, st)) != cudaSuccess)
+    else if (!a.fin.out &&
+             (e = cudaMemsetAsync(a.tile_counter, 0, sizeof(uint32_t) * kTileMaxPasses, st)) != cudaSuccess)
         return e;
     size_t off = 0;
     for (size_t p = 0; p < ts.progs.size(); ++p) {
@@ -1042,6 +1066,39 @@ cudaError_t launch_hv(const pned_model *m, const HvArgs &a, int nblocks, cudaStr
     }
 }
 
+// Rows up to which the last block of the H.v kernel finishes the sums: the finish kernel's
+// single-block range, whose order of additions it keeps bit for bit (longer lists go through
+// two levels).  One column only: several columns take a block as many passes, and the finish
+// kernel is then as fast (N = 20, R = 4, 16 columns: 459 us a step against 360 us).
+constexpr int64_t kFinishInKernel = 2048;
+
+cudaError_t launch_hv_sums(const pned_model *m, const HvArgs &a, int nblocks, double2 *out, cudaStream_t st,
+                           const TpsTail *tail, bool *in_kernel)
+{
+    const int64_t rows = hv_partials(m, a, nblocks);
+    const int kr = a.K * a.R;
+    const bool staged = a.R == 1 && !m->tprogs.empty() && m->use_tile && !find_xtiles(m, 1) && tile_staged(m);
+    HvArgs b = a;
+    const bool in = a.fin.done && kr == 1 && !staged && rows <= kFinishInKernel;
+    if (in_kernel) *in_kernel = in;
+    if (in) {
+        b.fin.base = a.partials;
+        b.fin.out = out;
+        b.fin.rows = int(rows);
+        b.fin.kr = kr;
+        b.fin.nctr = 0;
+        if (b.tile_counter) {   // counters that the last block leaves zero: no memset
+            b.tile_counter = b.fin.ctr;
+            b.fin.nctr = kTileCounters;
+        }
+        if (tail) b.tail = *tail;
+        return launch_hv(m, b, nblocks, st);
+    }
+    b.fin.out = nullptr;
+    cudaError_t e = launch_hv(m, b, nblocks, st);
+    return e == cudaSuccess ? launch_finish(a.partials, int(rows), kr, out, st) : e;
+}
+
 // First level of a long finish: block b sums rows [b * chunk, (b + 1) * chunk) of
 // partials ([row][KR]) in a fixed order and writes the sum over row b * chunk, the
 // first of its own rows, which no other block reads.
@@ -1092,10 +1149,11 @@ cudaError_t launch_dot(const pned_ctx *c, const double2 *x1, const double2 *x2, 
 }
 
 cudaError_t launch_residual(const pned_ctx *c, const double2 *W, const double2 *C, double2 *Rn, const double *sc,
-                            const double2 *alpha, cudaStream_t st)
+                            const double2 *alpha, double2 *out, const LanczosTail &tail, cudaStream_t st)
 {
+    const Finish fin{c->partials, out, c->fin_ctr, nullptr, c->nblocks, c->R, 0};
     residual_kernel<<<c->nblocks, kThreads, 0, st>>>(W, C, Rn, sc, alpha, c->m->dim, c->R, pick_vpt(c->R),
-                                                     c->partials);
+                                                     c->partials, fin, tail);
     return cudaGetLastError();
 }
 
@@ -1481,6 +1539,7 @@ extern "C" int pned_model_set_plan(pned_model *m, int R, const pned_tile_plan *p
     if (plan && (plan->max_passes > kTileMaxPasses || plan->window_bits > 30 || plan->row_fixed_bits > 8 ||
                  plan->j_bits > kTileMaxJB || plan->j_bits == 0 || plan->objective > 1 || plan->terms_in_flight > 2))
         return fail(PNED_EINVAL, "pned_model_set_plan: plan out of range");
+    cudaSetDevice(m->device);
     if (R == 1) {
         m->plan1 = plan ? *plan : pned_tile_plan{-1, -1, -1, -1, -1, -1, -1, -1, -1};
         m->plan1_set = plan != nullptr;
@@ -1575,11 +1634,17 @@ extern "C" int pned_ctx_create(pned_model *m, int R, size_t budget, pned_ctx **o
     c->partials_cap = int64_t(pslots);
     e = cudaMalloc(&c->partials, pbytes);
     if (e == cudaSuccess) e = cudaMalloc(&c->tile_ctr, sizeof(uint32_t) * kTileCounters);
+    if (e == cudaSuccess) e = cudaMalloc(&c->fin_ctr, sizeof(uint32_t) * (1 + kTileCounters));
+    if (e == cudaSuccess) e = cudaMemset(c->fin_ctr, 0, sizeof(uint32_t) * (1 + kTileCounters));
     if (e == cudaSuccess) e = cudaMalloc(&c->sums, sizeof(double2) * kMaxK * kMaxR * 4);
     if (e == cudaSuccess) e = cudaMalloc(&c->scal, sizeof(double) * kScalSlots * kMaxR);
-    if (e == cudaSuccess) e = cudaMallocHost(&c->h_sums, sizeof(double2) * kMaxK * kMaxR * 4);
+    if (e == cudaSuccess) e = cudaMallocHost(&c->h_sums, sizeof(double2) * (kMaxK * kMaxR * 4 + 1));
     if (e == cudaSuccess) e = cudaMalloc(&c->flag, sizeof(int) * 4);
     if (e == cudaSuccess) e = cudaMemset(c->flag, 0, sizeof(int) * 4);
+    if (e == cudaSuccess) {   // the scale of plain products: ones, never written again
+        const std::vector<double> ones(kMaxR, 1.0);
+        e = cudaMemcpy(slot(c.get(), kSlotOne), ones.data(), sizeof(double) * kMaxR, cudaMemcpyHostToDevice);
+    }
     if (e != cudaSuccess) {
         pned_ctx_destroy(c.release());
         return cuda_fail(e, "pned_ctx_create: scratch");
@@ -1602,6 +1667,7 @@ extern "C" int pned_ctx_destroy(pned_ctx *c)
     for (int k = 0; k < kMaxBuffers; ++k) cudaFree(c->buf[k]);
     cudaFree(c->partials);
     cudaFree(c->tile_ctr);
+    cudaFree(c->fin_ctr);
     cudaFree(c->sums);
     cudaFree(c->scal);
     cudaFree(c->flag);
@@ -1662,10 +1728,14 @@ int stage_in(pned_ctx *c, const pned_c128 *src, int flags, int k, const double2 
 
 int sums_to_host(pned_ctx *c, int KR)
 {
+    // the sums and the kernel error flag in one wait (the flag behind the sums, in pinned memory)
+    int *h_flag = reinterpret_cast<int *>(c->h_sums + kMaxK * kMaxR * 4);
+    *h_flag = 0;
     cudaError_t e = cudaMemcpyAsync(c->h_sums, c->sums, sizeof(double2) * KR, cudaMemcpyDeviceToHost, c->stream);
+    if (e == cudaSuccess) e = cudaMemcpyAsync(h_flag, c->flag, sizeof(int), cudaMemcpyDeviceToHost, c->stream);
     if (e == cudaSuccess) e = cudaStreamSynchronize(c->stream);
     if (e != cudaSuccess) return cuda_fail(e, "reading reduction results");
-    return check_kernel_flag(c);
+    return *h_flag ? check_kernel_flag(c) : PNED_OK;
 }
 
 // PNED_ETIMEOUT (and the flag cleared) if a kernel's bounded wait gave up.
@@ -1707,8 +1777,6 @@ extern "C" int pned_hv(pned_ctx *c, const pned_c128 *v1, pned_c128 *v0, double e
     rc = stage_in(c, v0, flags, 1, &dv0c);
     if (rc) return rc;
     double2 *dv0 = const_cast<double2 *>(dv0c);
-    rc = set_slot(c, kSlotOne, 1.0);
-    if (rc) return rc;
     HvArgs a{};
     a.C = dv1; a.P = dv0; a.W = dv0;
     a.sc = slot(c, kSlotOne); a.pc = slot(c, kSlotOne);
@@ -1717,9 +1785,7 @@ extern "C" int pned_hv(pned_ctx *c, const pned_c128 *v1, pned_c128 *v0, double e
     a.dim = c->m->dim; a.R = c->R; a.K = 1;
     a.err = c->flag;
     ctx_tile_args(c, a);
-    cudaError_t e = launch_hv(c->m, a, c->nblocks, c->stream);
-    if (e == cudaSuccess)
-        e = launch_finish(c->partials, int(hv_partials(c->m, a, c->nblocks)), c->R, c->sums, c->stream);
+    cudaError_t e = launch_hv_sums(c->m, a, c->nblocks, c->sums, c->stream);
     if (e != cudaSuccess) return cuda_fail(e, "pned_hv launch");
     if (!(flags & PNED_PTR_DEVICE)) {
         e = cudaMemcpyAsync(v0, dv0, sizeof(double2) * size_t(c->m->dim) * c->R, cudaMemcpyDeviceToHost, c->stream);

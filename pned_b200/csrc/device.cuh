@@ -11,6 +11,22 @@
 
 #include "kernels.cuh"
 
+namespace pned {
+// Device memory that a model's programs own.
+struct DevBuf {
+    void *p = nullptr;
+    DevBuf() = default;
+    DevBuf(const DevBuf &) = delete;
+    DevBuf &operator=(const DevBuf &) = delete;
+    ~DevBuf() { cudaFree(p); }
+    bool upload(const void *src, size_t bytes)
+    {
+        if (cudaMalloc(&p, bytes ? bytes : 1) != cudaSuccess) { p = nullptr; cudaGetLastError(); return false; }
+        return cudaMemcpy(p, src, bytes, cudaMemcpyHostToDevice) == cudaSuccess;
+    }
+};
+}  // namespace pned
+
 struct pned_model {
     pned::HostProgram hp;
     int device = 0;
@@ -35,6 +51,7 @@ struct pned_model {
         std::vector<std::unique_ptr<pned::XTileProgram>> progs;
         int lr = 0;
         int groups = 0;   // partner tiles over all passes
+        pned::DevBuf mem; // the passes' table sources
     };
     std::map<int, XTileSet> xtiles;
     std::set<int> rtiles_set;   // R > 1 with an explicit plan for the multi-vector kernel
@@ -120,6 +137,8 @@ struct pned_ctx {
     double2 *partials = nullptr;   // [nblocks][kMaxK][kMaxR], or per-tile sums of the single-vector tile kernel
     int64_t partials_cap = 0;      // double2 slots at `partials`
     uint32_t *tile_ctr = nullptr;  // [kTileCounters] tile counters of the dynamic tile order
+    uint32_t *fin_ctr = nullptr;   // [1 + kTileCounters] block count and tile counters of the kernels that
+                                   // finish their sums themselves (zero between launches)
     double2 *sums = nullptr;       // [4][kMaxK*kMaxR]
     double *scal = nullptr;        // [kScalSlots][kMaxR]
     int *flag = nullptr;
@@ -165,6 +184,11 @@ int pick_vpt(int R);
 void session_release(pned_ctx *c);
 
 cudaError_t launch_hv(const pned_model *m, const HvArgs &a, int nblocks, cudaStream_t st);
+// H.v and its sums into out[K * R]: in the kernel where a.fin.done is given and the rows
+// are few, else by the finish kernels.  `tail`: what follows the sums when they are finished
+// in the kernel (*in_kernel is set then).
+cudaError_t launch_hv_sums(const pned_model *m, const HvArgs &a, int nblocks, double2 *out, cudaStream_t st,
+                           const TpsTail *tail = nullptr, bool *in_kernel = nullptr);
 // Raises a kernel's dynamic shared memory limit to 200 KB (once per kernel and device).
 cudaError_t allow_dynamic_smem(const void *kern, int device);
 // Device chosen by pned_set_device on this host thread.
@@ -240,12 +264,19 @@ inline void ctx_tile_args(const pned_ctx *c, HvArgs &a)
 {
     a.tile_counter = c->tile_ctr;
     a.partials_cap = c->partials_cap;
+    a.fin.done = c->fin_ctr;
+    a.fin.ctr = c->fin_ctr + 1;
 }
 cudaError_t launch_finish(const double2 *partials, int nb, int KR, double2 *out, cudaStream_t st);
 cudaError_t launch_dot(const pned_ctx *c, const double2 *x1, const double2 *x2, const double2 *alpha, int mode,
                        double2 *out, cudaStream_t st);
+// Residual and, in its last block, beta^2 into `out` and the Lanczos step's epilogue.
+struct LanczosTail {
+    double *sc, *pc, *alpha, *beta;
+    int *counter, *flag;
+};
 cudaError_t launch_residual(const pned_ctx *c, const double2 *W, const double2 *C, double2 *Rn, const double *sc,
-                            const double2 *alpha, cudaStream_t st);
+                            const double2 *alpha, double2 *out, const LanczosTail &tail, cudaStream_t st);
 cudaError_t launch_gaussian(const pned_ctx *c, uint64_t seed, bool normalise, double2 *v, cudaStream_t st);
 
 inline uint64_t splitmix64_host(uint64_t x)
@@ -361,6 +392,82 @@ __device__ __forceinline__ void block_reduce_store(double2 (&red)[K][VPT], int G
         for (int w = 0; w < nw; ++w) s = cadd(s, sm[w][k][r]);
         partials[(sl * K + k) * R + r] = s;
     }
+}
+
+// The block that finishes a kernel's sums (see Finish): called by every thread of every
+// block after its partial sums are stored; true in all threads of the one block that comes
+// last, with f.out written.  The rows are added in a fixed order, so the result does not
+// depend on which block is last.  s_fin: kThreads values of shared memory.
+__device__ __forceinline__ bool finish_last(const Finish &f, double2 *s_fin)
+{
+    if (!f.out) return false;
+    __shared__ uint32_t s_last;
+    __threadfence();   // the block's partial sums before its count
+    __syncthreads();
+    const int tid = int(threadIdx.x);
+    if (tid == 0) s_last = atomicAdd(f.done, 1u) == gridDim.x - 1u ? 1u : 0u;
+    __syncthreads();
+    if (!s_last) return false;
+    __threadfence();
+    const int kr = f.kr, G = kThreads / kr, g = tid / kr, c = tid - g * kr;
+    double2 s = make_double2(0.0, 0.0);
+    if (g < G) {
+#pragma unroll 4
+        for (int row = g; row < f.rows; row += G) s = cadd(s, __ldcg(f.base + size_t(row) * kr + c));
+    }
+    s_fin[tid] = s;
+    __syncthreads();
+    for (int w = kThreads / 2; w > 0; w >>= 1) {
+        if (w < G && g < w && g + w < G) s_fin[tid] = cadd(s_fin[tid], s_fin[tid + w * kr]);
+        __syncthreads();
+    }
+    if (tid < kr) f.out[tid] = s_fin[tid];
+    if (tid == 0) *f.done = 0;
+    for (int i = tid; i < f.nctr; i += kThreads) f.ctr[i] = 0;
+    __syncthreads();
+    return true;
+}
+
+// TPS step: alpha1 = Re<v|(L-H)v>, beta = ||(L-H)v||, coefficients as eval_phys_val; the
+// next scales.  s: the sums [4][R]; so: the observables' sums.
+__device__ __forceinline__ void tps_tail(const TpsTail &t, const double2 *s, int nobs, const double2 *so)
+{
+    const int k = *t.counter, R = t.R;
+    __syncthreads();
+    for (int r = int(threadIdx.x); r < R; r += int(blockDim.x)) {
+        const double a1 = s[0 * R + r].x;
+        const double be = sqrt(s[1 * R + r].x);
+        const double2 zero = make_double2(0.0, 0.0);
+        const double2 gw = t.first ? zero : s[2 * R + r], gv = t.first ? zero : s[3 * R + r];
+        t.alpha[(size_t)k * R + r] = t.L - a1;
+        t.beta[(size_t)k * R + r] = be;
+        double *cf = t.coef + ((size_t)k * R + r) * t.ncoef;
+        cf[0] = double(2 * (k + 1)) / a1;
+        cf[1] = t.L;
+        cf[2] = be;
+        cf[3] = t.L - a1;
+        cf[4] = t.L * gv.x - gw.x;   // Re(L <vg|v1> - <vg|v0>)
+        for (int o = 0; o < nobs; ++o) {
+            cf[5 + 2 * o] = so[(2 * o) * R + r].x;
+            cf[6 + 2 * o] = so[(2 * o + 1) * R + r].x;
+        }
+        t.gscp[r] = t.gsc[r];
+        t.gsc[r] = t.sc[r];
+        t.sc[r] = 1.0 / be;
+    }
+    __syncthreads();
+    if (threadIdx.x == 0) *t.counter = k + 1;
+}
+
+// End of an H.v kernel: every thread of every block, after its partial sums.
+__device__ __forceinline__ void hv_finish(const HvArgs &a, double2 *s_fin)
+{
+    if (finish_last(a.fin, s_fin) && a.tail.on) tps_tail(a.tail, a.fin.out, 0, nullptr);
+}
+__device__ __forceinline__ void hv_finish(const HvArgs &a)
+{
+    __shared__ double2 s_fin[kThreads];
+    hv_finish(a, s_fin);
 }
 
 __device__ __forceinline__ uint64_t splitmix64(uint64_t x)

@@ -732,7 +732,7 @@ int plan_tiles(const HostProgram &P, int tbits, int jb, int fixed, int window_bi
 namespace {
 
 // Tile bits (`size` of n, the `fixed` lowest among them) that hold the most
-// masks: greedy from every mask as the start, then exchanges of one bit while
+// masks: greedy from up to 12 masks as the start (spread over the list), then exchanges of one bit while
 // more masks come inside; ties go to the set that touches more masks.
 uint32_t tile_most_masks(const std::vector<uint32_t> &masks, int n, int size, int fixed)
 {
@@ -748,9 +748,11 @@ uint32_t tile_most_masks(const std::vector<uint32_t> &masks, int n, int size, in
     uint32_t best = 0;
     int bs = -1;
     std::vector<uint32_t> starts{low};
-    for (uint32_t m : masks)
-        if (__builtin_popcount(low | m) <= size && std::find(starts.begin(), starts.end(), low | m) == starts.end())
-            starts.push_back(low | m);
+    const size_t step = std::max<size_t>(1, masks.size() / 12);
+    for (size_t i = 0; i < masks.size(); i += step) {
+        const uint32_t t = low | masks[i];
+        if (__builtin_popcount(t) <= size && std::find(starts.begin(), starts.end(), t) == starts.end()) starts.push_back(t);
+    }
     for (uint32_t t : starts) {
         while (__builtin_popcount(t) < size) {
             int bb = -1, bv = -1;

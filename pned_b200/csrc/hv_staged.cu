@@ -861,6 +861,7 @@ __global__ void __launch_bounds__(kThreads, 2)
         mbar_wait(bar_v, phase ^ 1u);
         mbar_wait(bar_e, phase ^ 1u);
     }
+    if (prog.last) hv_finish(a);
 }
 
 void *tile_tma_encoder()
@@ -958,7 +959,8 @@ static cudaError_t launch_tile_tma_t(const pned_model *m, const HvArgs &a, int n
     const bool dyn = tile_dynamic(m, a, nblocks);
     HvArgs b = a;
     if (!dyn) b.tile_counter = nullptr;
-    else if ((e = cudaMemsetAsync(a.tile_counter, 0, sizeof(uint32_t) * kTileMaxPasses, st)) != cudaSuccess)
+    else if (!a.fin.out &&
+             (e = cudaMemsetAsync(a.tile_counter, 0, sizeof(uint32_t) * kTileMaxPasses, st)) != cudaSuccess)
         return e;
     size_t off = 0;
     for (size_t p = 0; p < m->tprogs.size(); ++p) {

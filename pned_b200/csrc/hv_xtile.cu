@@ -106,8 +106,8 @@ __device__ __forceinline__ void x_member(const uint4 &S, uint32_t base, uint32_t
 // SM: fp64 pipe 28 %, issue 46 %.  Hence the classes (60 masks become 40 row reads at
 // N = 24), the perfect hash (3 instructions for a coefficient index), members as one
 // 16-byte constant read fetched ahead, and the indexed jump.  Measured H.V against the
-// multi-vector kernel: N = 24, R = 16 with a field 18.6 -> 13.7 ms, R = 12 without
-// 12.0 -> 8.9 ms, N = 22, R = 2 0.69 -> 0.49 ms, N = 26, R = 4 21.5 -> 14.3 ms.
+// multi-vector kernel: N = 24, R = 16 with a field 18.6 -> 13.2 ms, R = 12 without
+// 12.0 -> 8.3 ms, N = 22, R = 2 0.69 -> 0.49 ms, N = 26, R = 4 21.5 -> 14.3 ms.
 // Measured and dropped: a second class in flight through cp.async (15.1 against 14.8 ms:
 // the address arithmetic costs more than the latency it hides).
 template <bool RC, bool RD, int K, bool SLOT>
@@ -288,6 +288,7 @@ __global__ void __launch_bounds__(kThreads, 2)
     }
     if (!ctr) red[0] = cscale(sc * hs, red[0]);
     if (!ctr) x_sums_store<K>(red, s_red, lr, R, ch, a.partials + size_t(blk) * K * R);
+    if (prog.last) hv_finish(a, smem);   // the tile buffer is free behind the first barrier in there
 }
 
 const pned_model::XTileSet *find_xtiles(const pned_model *m, int R)
@@ -310,15 +311,19 @@ bool ensure_xtiles(pned_model *m, int R, bool slot_tables)
 {
     const HostProgram &hp = m->hp;
     if (pick_vpt(R) == 0) return false;
-    // One vector: only for complex coefficients (Gamma, a field, slot couplings).  With real
-    // ones a member is half the products, and the gather and tensor-copy kernels are faster
-    // (N = 24: 0.69 against 0.75 ms; complex: 1.04 against 0.93 ms, N = 26: 4.20 against 3.74 ms).
-    if (R == 1 && m->real_coef) return false;
+    // One vector: only for complex coefficients (Gamma, a field, slot couplings) -- with real
+    // ones a member is half the products, and the tensor-copy kernel is faster -- and only from
+    // 26 sites on (N = 26: 4.20 -> 3.63 ms, N = 28: 16.0 -> 15.1 ms).  Smaller bases keep the
+    // gather kernel's order of additions although it is slower (N = 24: 1.04 against 0.93 ms):
+    // the sign of the Ritz vector that vec12 finds turns on the last bit of alpha and beta, so
+    // another order may return -x where a caller had x.
+    if (R == 1 && (m->real_coef || hp.n < kTileBigSites)) return false;
     std::lock_guard<std::mutex> lock(m->rtiles_mu);
     if (m->xtiles.count(R)) return !m->xtiles[R].progs.empty();
     pned_model::XTileSet &xs = m->xtiles[R];
     std::vector<XTilePass> ps;
     if (plan_xtiles_for(hp, R, xs.lr, ps) != PNED_OK) return false;
+    std::vector<uint16_t> tsrc;   // of all passes
     for (size_t p = 0; p < ps.size(); ++p) {
         const XTilePass &t = ps[p];
         if (t.subs.size() > size_t(kMaxTerms)) { xs.progs.clear(); return false; }
@@ -328,7 +333,7 @@ bool ensure_xtiles(pned_model *m, int R, bool slot_tables)
         T->nsub = int(t.subs.size());
         T->nout = t.nout;
         T->ntab = int(t.tsrc.size());
-        for (size_t i = 0; i < t.tsrc.size(); ++i) T->tsrc[i] = uint16_t(t.tsrc[i] < 0 ? 0xffff : t.tsrc[i]);
+        for (int x : t.tsrc) tsrc.push_back(uint16_t(x < 0 ? 0xffff : x));
         T->nouter = int(t.outer.size());
         T->first = p == 0;
         T->last = p + 1 == ps.size();
@@ -344,6 +349,12 @@ bool ensure_xtiles(pned_model *m, int R, bool slot_tables)
         }
         xs.groups += t.groups;
         xs.progs.push_back(std::move(T));
+    }
+    if (!xs.mem.upload(tsrc.data(), sizeof(uint16_t) * tsrc.size())) { xs.progs.clear(); return false; }
+    const uint16_t *src = static_cast<const uint16_t *>(xs.mem.p);
+    for (auto &T : xs.progs) {
+        T->tsrc = src;
+        src += T->ntab;
     }
     // two blocks' shared memory per SM
     if (2 * (xtile_smem(m, xs, slot_tables) + 5 * 1024) > 227 * 1024) { xs.progs.clear(); return false; }
@@ -395,7 +406,8 @@ static cudaError_t launch_xtile_t(const pned_model *m, const pned_model::XTileSe
     const bool dyn = tile_dynamic(m, a, nblocks);
     HvArgs b = a;
     if (!dyn) b.tile_counter = nullptr;
-    else if ((e = cudaMemsetAsync(a.tile_counter, 0, sizeof(uint32_t) * xs.progs.size() * nch, st)) != cudaSuccess)
+    else if (!a.fin.out &&
+             (e = cudaMemsetAsync(a.tile_counter, 0, sizeof(uint32_t) * xs.progs.size() * nch, st)) != cudaSuccess)
         return e;
     size_t off = 0;
     for (size_t p = 0; p < xs.progs.size(); ++p) {

@@ -87,7 +87,9 @@ struct XTileProgram {
     uint32_t jexp[1 << kXJB];         // global bits of the thread's j-th state
     uint8_t rowpos[8];
     uint8_t outer[32];
-    uint16_t tsrc[kXMaxTab];          // table entry -> entry of the model's table (0xffff: zero)
+    const uint16_t *tsrc;             // table entry -> entry of the model's table (0xffff: zero), in global
+                                      // memory: read from the constant bank, each thread its own entry, it
+                                      // cost a block 10 us
     uint4 s[kMaxTerms + 1];           // members (XSub), one more read ahead
 };
 
@@ -103,6 +105,27 @@ struct TmaGeom {
     int lo[kTmaMaxRank] = {};      // lowest global bit of the dimension
     int nbits[kTmaMaxRank] = {};   // its bits
     int tile[kTmaMaxRank] = {};    // 1: tile bits (box spans it), 0: outer bits (box of 1)
+};
+
+// Sums finished by the kernel that wrote the last partial sums: its last block (counted
+// at `done`) adds rows of `base` ([rows][kr]) in a fixed order into out[kr].  out null:
+// separate finish kernels follow.  `done` and the tile counters are left zero for the
+// next launch.
+struct Finish {
+    const double2 *base;
+    double2 *out;
+    uint32_t *done;
+    uint32_t *ctr;
+    int rows, kr, nctr;
+};
+
+// Step epilogue of a TPS session, run behind the sums (see tps_tail).
+struct TpsTail {
+    int on, R, ncoef;
+    double L;
+    double *sc, *gsc, *gscp, *alpha, *beta, *coef;
+    int *counter;
+    int first;
 };
 
 // Per-call scalars: W = pc_r * P + sc_r * (H - shift) (sc_r * C); all from device memory.
@@ -135,6 +158,9 @@ struct HvArgs {
     // written per tile ([tile][K]) instead of per block.  Null: the static
     // order (tile = block + k * grid) with per-block sums.
     uint32_t *tile_counter;
+    // sums finished in the kernel (last pass), and what follows them
+    Finish fin;
+    TpsTail tail;
     int64_t partials_cap;   // double2 slots available at `partials` (per-tile sums need sum(tiles) * K)
     int rv_chunk;           // multi-vector kernel, dynamic order: tiles per chunk (set by the launcher)
     // Sz sector (set by launch_hv from the model): index -> state, and the Lin

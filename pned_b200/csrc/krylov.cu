@@ -19,60 +19,10 @@ namespace pned {
 // step epilogues (one block, one thread per vector)
 // ---------------------------------------------------------------------------
 
-// Lanczos: alpha = Re(sum0), beta = sqrt(sum1); record; next scales.
-__global__ void lanczos_epilogue(const double2 *__restrict__ sa, const double2 *__restrict__ sb, int R,
-                                 double *sc, double *pc, double *d_alpha, double *d_beta, int *counter,
-                                 int *flag)
+// TPS step whose sums the finish kernels made, and observables.
+__global__ void tps_epilogue(const TpsTail t, const double2 *__restrict__ s, int nobs, const double2 *__restrict__ so)
 {
-    __shared__ int k;
-    if (threadIdx.x == 0) k = *counter;
-    __syncthreads();
-    const int r = threadIdx.x;
-    if (r < R) {
-        const double al = sa[r].x;
-        const double be = sqrt(sb[r].x);
-        d_alpha[(size_t)k * R + r] = al;
-        d_beta[(size_t)k * R + r] = be;
-        if (!(be >= 0.5e-30)) atomicOr(flag, 1);
-        const double old = sc[r];
-        sc[r] = 1.0 / be;
-        pc[r] = -be * old;
-    }
-    __syncthreads();
-    if (threadIdx.x == 0) *counter = k + 1;
-}
-
-// TPS: alpha1 = Re<v|(L-H)v>, beta = ||(L-H)v||, coef as eval_phys_val.
-__global__ void tps_epilogue(const double2 *__restrict__ s, int R, int nobs, const double2 *__restrict__ so, double L,
-                             double *sc, double *gsc, double *gscp, double *d_alpha, double *d_beta, double *d_coef,
-                             int ncoef, int *counter)
-{
-    __shared__ int k;
-    if (threadIdx.x == 0) k = *counter;
-    __syncthreads();
-    const int r = threadIdx.x;
-    if (r < R) {
-        const double a1 = s[0 * R + r].x;
-        const double be = sqrt(s[1 * R + r].x);
-        const double2 gw = s[2 * R + r], gv = s[3 * R + r];
-        d_alpha[(size_t)k * R + r] = L - a1;
-        d_beta[(size_t)k * R + r] = be;
-        double *cf = d_coef + ((size_t)k * R + r) * ncoef;
-        cf[0] = double(2 * (k + 1)) / a1;
-        cf[1] = L;
-        cf[2] = be;
-        cf[3] = L - a1;
-        cf[4] = L * gv.x - gw.x;   // Re(L <vg|v1> - <vg|v0>)
-        for (int o = 0; o < nobs; ++o) {
-            cf[5 + 2 * o] = so[(2 * o) * R + r].x;
-            cf[6 + 2 * o] = so[(2 * o + 1) * R + r].x;
-        }
-        gscp[r] = gsc[r];
-        gsc[r] = sc[r];
-        sc[r] = 1.0 / be;
-    }
-    __syncthreads();
-    if (threadIdx.x == 0) *counter = k + 1;
+    tps_tail(t, s, nobs, so);
 }
 
 // Diagonal observables: <v|O v> and <g|O v>, v = sc C, g = gsc G.
@@ -214,22 +164,47 @@ __global__ void dsf_start_epilogue(const double2 *__restrict__ s, int R, int n, 
     }
 }
 
-// x += a p ; r -= a y    (complex a, one vector)
-__global__ void cg_update_xr(double2 *x, double2 *r, const double2 *__restrict__ p, const double2 *__restrict__ y,
-                             double2 a, int64_t n)
+// Scalars of a CG solve on the device.
+enum : int { kCgPr = 0 /* <p|r> */, kCgPy /* <p|y> */, kCgRr0 /* <r|r> before the update */, kCgRr /* after */, kCgN };
+
+// x += a p ; r -= a y, a = <p|r> / <p|y> (one vector); <r|r> into s[kCgRr] by the last block.
+// The scalars stay on the device: an iteration is three kernels behind the H.v's and no
+// host round trip (it was four dot products, each with a finish kernel and two waits).
+__global__ void __launch_bounds__(kThreads) cg_update_xr(double2 *x, double2 *r, const double2 *__restrict__ p,
+                                                         const double2 *__restrict__ y, const double2 *s, int64_t n,
+                                                         double2 *partials, const Finish fin)
 {
+    const double2 pr = s[kCgPr], py = s[kCgPy];
+    const double den = py.x * py.x + py.y * py.y;
+    const double2 a = make_double2((pr.x * py.x + pr.y * py.y) / den, (pr.y * py.x - pr.x * py.y) / den);
+    double2 red[1][1] = {{make_double2(0.0, 0.0)}};
     for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
         x[i] = cfma(a, p[i], x[i]);
-        const double2 ay = cmul(a, y[i]);
-        r[i] = make_double2(r[i].x - ay.x, r[i].y - ay.y);
+        const double2 ay = cmul(a, y[i]), ro = r[i];
+        const double2 rn = make_double2(ro.x - ay.x, ro.y - ay.y);
+        r[i] = rn;
+        red[0][0].x += rn.x * rn.x + rn.y * rn.y;
     }
+    block_reduce_store<1, 1>(red, 1, 1, 1, partials);
+    __shared__ double2 s_fin[kThreads];
+    finish_last(fin, s_fin);
 }
 
-// p = r + b p
-__global__ void cg_update_p(double2 *p, const double2 *__restrict__ r, double b, int64_t n)
+// p = r + b p, b = <r|r> / <r|r> before; <p|r> into s[kCgPr] and s[kCgRr0] <- s[kCgRr] by the last block.
+__global__ void __launch_bounds__(kThreads) cg_update_p(double2 *p, const double2 *__restrict__ r, double2 *s, int64_t n,
+                                                        double2 *partials, const Finish fin)
 {
-    for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x)
-        p[i] = make_double2(r[i].x + b * p[i].x, r[i].y + b * p[i].y);
+    const double b = s[kCgRr].x / s[kCgRr0].x;
+    double2 red[1][1] = {{make_double2(0.0, 0.0)}};
+    for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
+        const double2 ri = r[i], po = p[i];
+        const double2 pn = make_double2(ri.x + b * po.x, ri.y + b * po.y);
+        p[i] = pn;
+        red[0][0] = cadd(red[0][0], cconjmul(pn, ri));
+    }
+    block_reduce_store<1, 1>(red, 1, 1, 1, partials);
+    __shared__ double2 s_fin[kThreads];
+    if (finish_last(fin, s_fin) && threadIdx.x == 0) s[kCgRr0] = s[kCgRr];
 }
 
 __global__ void scale_real_kernel(double2 *v, double f, int64_t n)
@@ -303,17 +278,11 @@ static cudaError_t lanczos_step(pned_ctx *c, Session &S, bool first)
     ctx_tile_args(c, a);
     double2 *sa = c->sums, *sb = c->sums + kMaxK * kMaxR;
     if (S.ev_hv0) cudaEventRecord(S.ev_hv0, c->stream);
-    cudaError_t e = launch_hv(c->m, a, c->nblocks, c->stream);
+    cudaError_t e = launch_hv_sums(c->m, a, c->nblocks, sa, c->stream);
     if (S.ev_hv1) cudaEventRecord(S.ev_hv1, c->stream);
-    if (e == cudaSuccess) e = launch_finish(c->partials, int(hv_partials(c->m, a, c->nblocks)), R, sa, c->stream);
+    const LanczosTail tail{slot(c, kSlotSc), slot(c, kSlotPc), S.d_alpha, S.d_beta, S.d_counter, S.d_flag};
     if (e == cudaSuccess)
-        e = launch_residual(c, c->buf[S.b2], c->buf[S.b0], c->buf[S.b1], slot(c, kSlotSc), sa, c->stream);
-    if (e == cudaSuccess) e = launch_finish(c->partials, c->nblocks, R, sb, c->stream);
-    if (e == cudaSuccess) {
-        lanczos_epilogue<<<1, 32 * ((R + 31) / 32), 0, c->stream>>>(sa, sb, R, slot(c, kSlotSc), slot(c, kSlotPc),
-                                                                   S.d_alpha, S.d_beta, S.d_counter, S.d_flag);
-        e = cudaGetLastError();
-    }
+        e = launch_residual(c, c->buf[S.b2], c->buf[S.b0], c->buf[S.b1], slot(c, kSlotSc), sa, sb, tail, c->stream);
     std::swap(S.b0, S.b1);
     return e;
 }
@@ -334,11 +303,12 @@ static cudaError_t tps_step(pned_ctx *c, Session &S, bool first)
     a.err = c->flag;
     ctx_tile_args(c, a);
     if (S.ev_hv0) cudaEventRecord(S.ev_hv0, c->stream);
-    cudaError_t e = launch_hv(c->m, a, c->nblocks, c->stream);
+    const TpsTail tail{1, R, S.ncoef, S.L, slot(c, kSlotSc), slot(c, kSlotGsc), slot(c, kSlotGscPrev), S.d_alpha,
+                       S.d_beta, S.d_coef, S.d_counter, first ? 1 : 0};
+    bool closed = false;   // the H.v kernel closes the step (no observables)
+    cudaError_t e = launch_hv_sums(c->m, a, c->nblocks, c->sums, c->stream, S.nobs ? nullptr : &tail, &closed);
+    closed = closed && !S.nobs;
     if (S.ev_hv1) cudaEventRecord(S.ev_hv1, c->stream);
-    if (e == cudaSuccess)
-        e = launch_finish(c->partials, int(hv_partials(c->m, a, c->nblocks)), 4 * R, c->sums, c->stream);
-    if (first && e == cudaSuccess) e = cudaMemsetAsync(c->sums + 2 * R, 0, sizeof(double2) * 2 * R, c->stream);
     for (int o = 0; o < S.nobs && e == cudaSuccess; ++o) {
         const DevObs &ob = S.obs[o];
         obs_kernel<<<c->nblocks, kThreads, 0, c->stream>>>(c->buf[S.b0], first ? nullptr : c->buf[S.b2],
@@ -348,10 +318,8 @@ static cudaError_t tps_step(pned_ctx *c, Session &S, bool first)
         e = cudaGetLastError();
         if (e == cudaSuccess) e = launch_finish(c->partials, c->nblocks, 2 * R, S.d_osum + 2 * o * R, c->stream);
     }
-    if (e == cudaSuccess) {
-        tps_epilogue<<<1, 32 * ((R + 31) / 32), 0, c->stream>>>(c->sums, R, S.nobs, S.d_osum, S.L, slot(c, kSlotSc),
-                                                               slot(c, kSlotGsc), slot(c, kSlotGscPrev), S.d_alpha,
-                                                               S.d_beta, S.d_coef, S.ncoef, S.d_counter);
+    if (e == cudaSuccess && !closed) {
+        tps_epilogue<<<1, 32 * ((R + 31) / 32), 0, c->stream>>>(tail, c->sums, S.nobs, S.d_osum);
         e = cudaGetLastError();
     }
     const int og = S.b2;
@@ -869,7 +837,6 @@ extern "C" int pned_cg_run(pned_ctx *c, double E, const pned_c128 *b_init, int i
                                     (flags & PNED_PTR_DEVICE) ? cudaMemcpyDeviceToDevice : cudaMemcpyHostToDevice,
                                     c->stream);
     if (e != cudaSuccess) return cuda_fail(e, "pned_cg_run: staging b");
-    if ((rc = set_slot(c, kSlotOne, 1.0))) return rc;
     const int nb = c->nblocks;
     auto dot = [&](const double2 *u, const double2 *v, double2 &out) -> int {
         cudaError_t err = launch_dot(c, u, v, nullptr, 0, c->sums, c->stream);
@@ -878,14 +845,17 @@ extern "C" int pned_cg_run(pned_ctx *c, double E, const pned_c128 *b_init, int i
         out = c->h_sums[0];
         return q;
     };
+    double2 *s = c->sums;   // the solve's scalars (kCgN)
+    auto fin = [&](double2 *out) { return Finish{c->partials, out, c->fin_ctr, nullptr, nb, 1, 0}; };
     bool cg_loop_saved = false;   // the SAVEd `loop` flag of cg1 (S1/2 cg.f90:118)
     int total_cg = 0, itr_inv = 0;
     for (int it = 1; it <= inv_max; ++it) {
         itr_inv = it;
-        // ---- cg1: solve (H - E) x = b
+        // ---- cg1: solve (H - E) x = b; r = p = b, so <p|r> = <r|r> = <b|b>
         double2 bc;
         if ((rc = dot(b, b, bc))) return rc;
-        e = cudaMemcpyAsync(r, b, bytes, cudaMemcpyDeviceToDevice, c->stream);
+        e = cudaMemcpyAsync(s + kCgRr0, s, sizeof(double2), cudaMemcpyDeviceToDevice, c->stream);
+        if (e == cudaSuccess) e = cudaMemcpyAsync(r, b, bytes, cudaMemcpyDeviceToDevice, c->stream);
         if (e == cudaSuccess) e = cudaMemcpyAsync(p, b, bytes, cudaMemcpyDeviceToDevice, c->stream);
         if (e == cudaSuccess) e = cudaMemsetAsync(x, 0, bytes, c->stream);
         if (e != cudaSuccess) return cuda_fail(e, "cg init");
@@ -900,19 +870,15 @@ extern "C" int pned_cg_run(pned_ctx *c, double E, const pned_c128 *b_init, int i
             a.dim = n; a.R = 1; a.K = 1;
             a.err = c->flag;
             ctx_tile_args(c, a);
-            e = launch_hv(c->m, a, nb, c->stream);
+            e = launch_hv_sums(c->m, a, nb, s + kCgPy, c->stream);   // y and <p|y>
             if (e != cudaSuccess) return cuda_fail(e, "cg hv");
-            double2 crp, cyp, rc1, rc2;
-            if ((rc = dot(p, r, crp)) || (rc = dot(p, y, cyp)) || (rc = dot(r, r, rc1))) return rc;
-            const double den = cyp.x * cyp.x + cyp.y * cyp.y;
-            const double2 al = make_double2((crp.x * cyp.x + crp.y * cyp.y) / den, (crp.y * cyp.x - crp.x * cyp.y) / den);
-            cg_update_xr<<<nb, kThreads, 0, c->stream>>>(x, r, p, y, al, n);
-            if ((rc = dot(r, r, rc2))) return rc;
-            const double beta = rc2.x / rc1.x;
-            cg_update_p<<<nb, kThreads, 0, c->stream>>>(p, r, beta, n);
+            cg_update_xr<<<nb, kThreads, 0, c->stream>>>(x, r, p, y, s, n, c->partials, fin(s + kCgRr));
+            cg_update_p<<<nb, kThreads, 0, c->stream>>>(p, r, s, n, c->partials, fin(s + kCgPr));
             e = cudaGetLastError();
             if (e != cudaSuccess) return cuda_fail(e, "cg update");
             if (k % 5 != 0) continue;
+            if ((rc = sums_to_host(c, kCgN))) return rc;
+            const double2 rc2 = c->h_sums[kCgRr];
             if (std::sqrt(std::hypot(rc2.x, rc2.y)) < 1.0e-9 * std::sqrt(std::hypot(bc.x, bc.y))) cg_loop_saved = true;
             if (cg_loop_saved) break;
         }

@@ -8,11 +8,10 @@
 // Per step (one CUDA graph per three steps, since buffer roles rotate P -> C -> W):
 //   slot_hv_kernel        W = pc P + hsc (H_r - shift) C  with per-slot tables and
 //                         diagonal; sums <v|hv>, ||W||^2, <g|W>, <g|v>
-//   finish                4R sums
+//                         (4R sums: in its last block, or the finish kernels)
 //   slot_residual_kernel  Lanczos slots: W <- W - Re(alpha) v, beta^2 = ||W - alpha v||^2;
 //                         eigenvector slots also accumulate x += c_k v
-//   finish                R sums
-//   slot_epilogue         per-slot alpha/beta/TPS coefficients and next scales
+//                         its last block: R sums, then slot_epilogue: per-slot alpha/beta/TPS coefficients and next scales
 // Lanczos follows S_one_half/Hybrid_TPS_Lanczos.f90:48-163 (alpha from the H.v
 // product, beta through the complex alpha, update with the real alpha), TPS
 // follows S_one_half/Hybrid_TPS_TPS.f90:325-409 and eval_phys_val :83-111, the
@@ -122,16 +121,72 @@ __global__ void __launch_bounds__(kThreads, 2) slot_hv_kernel(const __grid_const
 struct SlotResArgs {
     double2 *W;
     const double2 *C;
-    const double *cf;
+    double *cf;
     const double2 *sums;     // [4][R] from the H.V pass
     SlotDev *st;
-    const double *hist_a;    // [R][max_steps]
+    double *hist_a, *hist_b, *coef;   // [R][max_steps] (coef: 5 a step)
+    Finish fin;              // beta^2 per slot
     double2 *partials;       // [nblocks][1][R]
     int64_t dim;
     int R, max_steps;
 };
 
-// Lanczos residual per slot (see the file comment); other slots are not touched.
+__device__ __forceinline__ void slot_idle(double *cf, int R, int r)
+{
+    for (int f = 0; f < kCf; ++f) cf[f * R + r] = 0.0;
+}
+
+// Records the step of every active slot and sets the next step's scales.
+__device__ void slot_epilogue(const double2 *s4, const double2 *sb, int R, SlotDev *st, double *cf, double *hist_a,
+                              double *hist_b, double *coef, int max_steps)
+{
+    const int r = threadIdx.x;
+    if (r >= R) return;
+    SlotDev &d = st[r];
+    if (!d.active) { slot_idle(cf, R, r); return; }
+    const int k = d.counter;
+    const double sc_old = cf[kCfSc * R + r];
+    const size_t h = size_t(r) * max_steps + k;
+    double be;
+    if (d.kind == PNED_SLOT_TPS) {
+        const double a1 = s4[0 * R + r].x;
+        be = sqrt(s4[1 * R + r].x);
+        const double2 gw = s4[2 * R + r], gv = s4[3 * R + r];
+        hist_a[h] = d.L - a1;
+        hist_b[h] = be;
+        double *c = coef + h * 5;
+        c[0] = double(2 * (k + 1)) / a1;
+        c[1] = d.L;
+        c[2] = be;
+        c[3] = d.L - a1;
+        c[4] = d.L * gv.x - gw.x;
+        cf[kCfGsc * R + r] = sc_old;
+        cf[kCfSc * R + r] = 1.0 / be;
+        cf[kCfHsc * R + r] = -1.0 / be;
+        cf[kCfShift * R + r] = d.L;
+        cf[kCfPc * R + r] = 0.0;
+    } else {
+        if (d.kind == PNED_SLOT_LANCZOS) {
+            be = sqrt(sb[r].x);
+            hist_a[h] = s4[r].x;
+            hist_b[h] = be;
+        } else {
+            be = hist_b[h];
+        }
+        cf[kCfPc * R + r] = -be * sc_old;
+        cf[kCfSc * R + r] = 1.0 / be;
+        cf[kCfHsc * R + r] = 1.0 / be;
+        cf[kCfShift * R + r] = 0.0;
+        cf[kCfGsc * R + r] = 0.0;
+    }
+    d.counter = k + 1;
+    if (!(be >= 0.5e-30)) { d.status = 1; d.active = 0; }
+    if (d.counter >= d.target) d.active = 0;
+    if (!d.active) slot_idle(cf, R, r);
+}
+
+// Lanczos residual per slot (see the file comment); other slots are not touched.  The last
+// block adds the blocks' sums and closes the step.
 template <int VPT>
 __global__ void __launch_bounds__(kThreads) slot_residual_kernel(const SlotResArgs a)
 {
@@ -190,60 +245,9 @@ __global__ void __launch_bounds__(kThreads) slot_residual_kernel(const SlotResAr
         }
     }
     block_reduce_store<1, VPT>(red, G, VPT, R, a.partials);
-}
-
-__device__ __forceinline__ void slot_idle(double *cf, int R, int r)
-{
-    for (int f = 0; f < kCf; ++f) cf[f * R + r] = 0.0;
-}
-
-// Records the step of every active slot and sets the next step's scales.
-__global__ void slot_epilogue(const double2 *__restrict__ s4, const double2 *__restrict__ sb, int R, SlotDev *st,
-                              double *cf, double *hist_a, double *hist_b, double *coef, int max_steps)
-{
-    const int r = threadIdx.x;
-    if (r >= R) return;
-    SlotDev &d = st[r];
-    if (!d.active) { slot_idle(cf, R, r); return; }
-    const int k = d.counter;
-    const double sc_old = cf[kCfSc * R + r];
-    const size_t h = size_t(r) * max_steps + k;
-    double be;
-    if (d.kind == PNED_SLOT_TPS) {
-        const double a1 = s4[0 * R + r].x;
-        be = sqrt(s4[1 * R + r].x);
-        const double2 gw = s4[2 * R + r], gv = s4[3 * R + r];
-        hist_a[h] = d.L - a1;
-        hist_b[h] = be;
-        double *c = coef + h * 5;
-        c[0] = double(2 * (k + 1)) / a1;
-        c[1] = d.L;
-        c[2] = be;
-        c[3] = d.L - a1;
-        c[4] = d.L * gv.x - gw.x;
-        cf[kCfGsc * R + r] = sc_old;
-        cf[kCfSc * R + r] = 1.0 / be;
-        cf[kCfHsc * R + r] = -1.0 / be;
-        cf[kCfShift * R + r] = d.L;
-        cf[kCfPc * R + r] = 0.0;
-    } else {
-        if (d.kind == PNED_SLOT_LANCZOS) {
-            be = sqrt(sb[r].x);
-            hist_a[h] = s4[r].x;
-            hist_b[h] = be;
-        } else {
-            be = hist_b[h];
-        }
-        cf[kCfPc * R + r] = -be * sc_old;
-        cf[kCfSc * R + r] = 1.0 / be;
-        cf[kCfHsc * R + r] = 1.0 / be;
-        cf[kCfShift * R + r] = 0.0;
-        cf[kCfGsc * R + r] = 0.0;
-    }
-    d.counter = k + 1;
-    if (!(be >= 0.5e-30)) { d.status = 1; d.active = 0; }
-    if (d.counter >= d.target) d.active = 0;
-    if (!d.active) slot_idle(cf, R, r);
+    __shared__ double2 s_fin[kThreads];
+    if (finish_last(a.fin, s_fin))
+        slot_epilogue(a.sums, a.fin.out, R, a.st, a.cf, a.hist_a, a.hist_b, a.coef, a.max_steps);
 }
 
 // Writes column r of C (a dense vector, or S^z_q of one), zeroes column r of P
@@ -356,7 +360,8 @@ struct pned_slots {
     double *vcoef = nullptr;         // [R][max_steps]
     double2 *partials = nullptr, *sums = nullptr, *scratch = nullptr;   // scratch: [R][n] phases + [R][nbond*4] dtab
     int64_t partials_cap = 0;        // double2 slots at `partials`
-    uint32_t *tile_ctr = nullptr;    // R = 1: tile counters of the single-vector kernel's dynamic order
+    uint32_t *tile_ctr = nullptr;    // tile counters of the dynamic tile order
+    uint32_t *fin_ctr = nullptr;     // block count and tile counters of kernels that finish their sums
     cudaGraphExec_t graph = nullptr;
     int64_t enqueued = 0;
     // R = 1: the batch's table and diagonal have the layout of a model's, so the
@@ -391,7 +396,7 @@ cudaError_t slot_step(pned_slots *S)
     const int R = S->R;
     double2 *P = S->buf[S->role[0]], *C = S->buf[S->role[1]], *W = S->buf[S->role[2]];
     cudaError_t e;
-    int nb_hv = S->nblocks;
+    double2 *s4 = S->sums, *sb = S->sums + 4 * kMaxR;
     if (S->tile) {
         HvArgs a{};
         a.C = C; a.P = P; a.W = W; a.G = P;
@@ -402,8 +407,9 @@ cudaError_t slot_step(pned_slots *S)
         a.slot_tables = R > 1;
         a.tile_counter = S->tile_ctr;
         a.partials_cap = S->partials_cap;
-        e = launch_hv(&S->tm, a, S->nblocks, S->stream);
-        nb_hv = int(hv_partials(&S->tm, a, S->nblocks));
+        a.fin.done = S->fin_ctr;
+        a.fin.ctr = S->fin_ctr + 1;
+        e = launch_hv_sums(&S->tm, a, S->nblocks, s4, S->stream);
     } else {
         SlotHvArgs a{};
         a.C = C; a.P = P; a.W = W;
@@ -415,12 +421,13 @@ cudaError_t slot_step(pned_slots *S)
         case 2: e = launch_slot_hv_v<2>(S, a); break;
         default: e = launch_slot_hv_v<1>(S, a); break;
         }
+        if (e == cudaSuccess) e = launch_finish(S->partials, S->nblocks, 4 * R, s4, S->stream);
     }
-    double2 *s4 = S->sums, *sb = S->sums + 4 * kMaxR;
-    if (e == cudaSuccess) e = launch_finish(S->partials, nb_hv, 4 * R, s4, S->stream);
     SlotResArgs b{};
-    b.W = W; b.C = C; b.cf = S->cf; b.sums = s4; b.st = S->st; b.hist_a = S->hist_a;
+    b.W = W; b.C = C; b.cf = S->cf; b.sums = s4; b.st = S->st; b.hist_a = S->hist_a; b.hist_b = S->hist_b;
+    b.coef = S->coef;
     b.partials = S->partials; b.dim = S->dim; b.R = R; b.max_steps = S->max_steps;
+    b.fin = Finish{S->partials, sb, S->fin_ctr, nullptr, S->nblocks, R, 0};
     if (e == cudaSuccess) {
         switch (pick_vpt(R)) {
         case 4: e = launch_slot_res_v<4>(S, b); break;
@@ -428,12 +435,6 @@ cudaError_t slot_step(pned_slots *S)
         case 2: e = launch_slot_res_v<2>(S, b); break;
         default: e = launch_slot_res_v<1>(S, b); break;
         }
-    }
-    if (e == cudaSuccess) e = launch_finish(S->partials, S->nblocks, R, sb, S->stream);
-    if (e == cudaSuccess) {
-        slot_epilogue<<<1, 32 * ((R + 31) / 32), 0, S->stream>>>(s4, sb, R, S->st, S->cf, S->hist_a, S->hist_b,
-                                                                 S->coef, S->max_steps);
-        e = cudaGetLastError();
     }
     // P <- C, C <- W, W <- P
     const int p = S->role[0];
@@ -457,6 +458,7 @@ void slots_free(pned_slots *S)
     cudaFree(S->diag); cudaFree(S->table); cudaFree(S->s1); cudaFree(S->s2); cudaFree(S->st); cudaFree(S->cf);
     cudaFree(S->hist_a); cudaFree(S->hist_b); cudaFree(S->coef); cudaFree(S->vcoef);
     cudaFree(S->partials); cudaFree(S->sums); cudaFree(S->scratch); cudaFree(S->tile_ctr);
+    cudaFree(S->fin_ctr);
     if (S->own_stream) cudaStreamDestroy(S->own_stream);
 }
 
@@ -622,6 +624,8 @@ extern "C" int pned_slots_create(const pned_model_desc *structure, int R, int ma
     S->partials_cap = std::max<int64_t>(S->partials_cap, (S->dim * R / 2048 + 1) * 2 * kMaxK * R / std::min(R, kXMaxVec));
     if (e == cudaSuccess) e = salloc(S.get(), &S->partials, size_t(S->partials_cap));
     if (e == cudaSuccess) e = cudaMalloc(&S->tile_ctr, sizeof(uint32_t) * kTileCounters);
+    if (e == cudaSuccess) e = cudaMalloc(&S->fin_ctr, sizeof(uint32_t) * (1 + kTileCounters));
+    if (e == cudaSuccess) e = cudaMemset(S->fin_ctr, 0, sizeof(uint32_t) * (1 + kTileCounters));
     if (e == cudaSuccess) e = salloc(S.get(), &S->sums, size_t(12) * kMaxR);
     if (e == cudaSuccess) e = salloc(S.get(), &S->scratch, size_t(R) * 64 + size_t(R) * S->nbond * 4);
     if (e == cudaSuccess) e = cudaMemcpy(S->s1, hp.dsite1.data(), sizeof(int) * S->nbond, cudaMemcpyHostToDevice);
@@ -853,7 +857,7 @@ extern "C" int pned_slots_set_plan(pned_slots *S, const pned_tile_plan *plan)
     if (plan) S->tm.carveout = plan->l1_carveout != 0;
     if (S->R == 1) {
         S->tm.plan1 = plan ? *plan : def;
-        S->tm.plan1_set = plan != nullptr;
+        S->tm.plan1_set = !plan_default(plan);
         build_tile_programs(&S->tm);
         S->tile = S->tm.use_tile;
     }

@@ -47,9 +47,9 @@ CANDIDATES_R = [(-1, -1, -1), (0, 6, 2), (0, 8, 2), (0, 10, 2), (1, 10, 2), (3, 
                 (0, 6, 2, -1, 1, 0, -1, 1), (0, 8, 2, -1, 1, 0, -1, 1), (0, 10, 2, -1, 1, 0, -1, 1),
                 (1, 8, 2, -1, 1, 0, -1, 1), (0, 8, 3, -1, 1, 0, -1, 1), (0, 12, 1, -1, 1, 0, -1, 1)]
 
-# the library's own default: from 2^18 states on, complex couplings run the class-tiled kernel
+# the library's own default: from 26 sites on, complex couplings run the class-tiled kernel
 DEFAULT = (-1, -1, -1, -1)
-DEFAULT_DIM = 1 << 18
+DEFAULT_DIM = 1 << 26
 
 _cache: dict = {}
 

@@ -765,3 +765,40 @@ def test_complex_diagonal_tile_kernels(plan):
     ref = v0.copy()
     prr = om.p_mltply_v3(v1, ref, 0.0625)
     assert rel(w, ref) <= 1e-12 and abs(pr[0] - prr) <= 1e-12 * abs(prr)
+
+
+def _chain_model(n, field):
+    """An open chain of n sites (odd n included) with the three bond types in turn."""
+    ipair = np.array([[i + 1, i + 2] for i in range(n - 1)], dtype=np.int32).reshape(-1)
+    bt = np.array([1 + i % 3 for i in range(n - 1)], dtype=np.int32)
+    X, skip, pt = P.build_xlocal(2, 0, KHGH if field else KH, field=FIELD if field else None)
+    return (P.Model(n, 2, 0, ipair, bt, X, skip, pt), O.Model(n, 2, 0, ipair, bt, X, skip, pt))
+
+
+@pytest.mark.parametrize("n,R,field", [(13, 1, False), (17, 2, True), (17, 6, False), (16, 4, True), (19, 8, True),
+                                       (15, 16, False), (17, 12, True)])
+def test_class_tiled_and_in_kernel_sums_parity(n, R, field):
+    """The class-tiled kernel (several vectors, from 2^18 elements on), odd site counts
+    included, and the sums that a kernel's last block finishes (one vector): H.V, prdct and
+    a short Lanczos chain as the oracle's, within the bounds of the other kernels.  Two
+    calls in a row: the counters that a kernel leaves for the next are zero."""
+    gm, om = _chain_model(n, field)
+    ctx = P.Context(gm, R=R)
+    rng = np.random.default_rng(n * 17 + R)
+    D = gm.dim
+    v1 = (rng.standard_normal((D, R)) + 1j * rng.standard_normal((D, R))).astype(np.complex128)
+    v0 = (0.2 * rng.standard_normal((D, R)) + 0.1j * rng.standard_normal((D, R))).astype(np.complex128)
+    for _ in range(2):
+        w = np.ascontiguousarray(v0).reshape(-1).copy()
+        pr = ctx.p_mltply_v3(np.ascontiguousarray(v1).reshape(-1), w, 0.0625)
+        w = w.reshape(D, R)
+        for r in range(R):
+            ref = np.ascontiguousarray(v0[:, r]).copy()
+            prr = om.p_mltply_v3(np.ascontiguousarray(v1[:, r]), ref, 0.0625)
+            assert rel(w[:, r], ref) <= 1e-12
+            assert abs(pr[r] - prr) <= 1e-12 * np.linalg.norm(v1[:, r]) * np.linalg.norm(ref)
+    V = v1 / np.linalg.norm(v1, axis=0)
+    out = ctx.lanczos(np.ascontiguousarray(V).reshape(-1), 8)
+    for r in (0, R - 1):
+        ref = om.lanczos(np.ascontiguousarray(V[:, r]), 8)
+        assert rel(out["alpha"][:, r], ref["alpha"]) <= 1e-10 and rel(out["beta"][:, r], ref["beta"]) <= 1e-10

@@ -319,8 +319,8 @@ def test_default_plan_below_26_sites_is_the_gather_plan():
     assert api.tile_plan_export(d) == api.tile_plan_export(d, 8, 10, -1, 3, objective=0)
 
 
-XTILE_CASES = [(14, 16, True), (16, 4, False), (18, 2, True), (18, 1, True), (18, 4, True), (18, 6, False), (20, 8, True),
-               (22, 1, True), (24, 12, False), (24, 16, True)]
+XTILE_CASES = [(14, 16, True), (16, 4, False), (18, 2, True), (26, 1, True), (18, 4, True), (18, 6, False), (20, 8, True),
+               (28, 1, False), (24, 12, False), (24, 16, True)]
 
 
 @pytest.mark.parametrize("n,R,field", XTILE_CASES)
