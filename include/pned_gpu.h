@@ -208,6 +208,16 @@ int pned_qtile_plan_export(const pned_model_desc *d, int k, int low, int64_t *ou
  */
 int pned_xtile_plan_export(const pned_model_desc *d, int R, int64_t *out, int64_t cap, int64_t *len);
 /*
+ * Test hook (no counterpart in the reference): the S = 1 passes for tiles of k
+ * sites (the `low` lowest in every tile).  out[0..cap) receives int64 values,
+ * *len the full count: n, the number of radix terms X, X records (offset, s1, s2,
+ * tab), the table size T and T flags (entry nonzero), the number of passes, and
+ * per pass (k, nouter, nmembers, ntab), sites[k] (the two J sites first),
+ * outer[nouter], nmembers records (loff, tab, var, first, sh1, sh2, m1, m2) and
+ * the source entry of each table entry.
+ */
+int pned_q3_plan_export(const pned_model_desc *d, int k, int low, int64_t *out, int64_t cap, int64_t *len);
+/*
  * Measurement hook (no counterpart in the reference): the partner-tile
  * staging the single-vector plan actually runs (0 gathered through L1/L2,
  * 1 cp.async, 2 bulk copies) and, for 2, the number of ring stages.

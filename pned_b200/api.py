@@ -471,6 +471,28 @@ def xtile_plan_export(desc: "ModelInput", R: int) -> dict:
     return {"lr": lr, "xterms": xterms, "passes": passes}
 
 
+def q3_plan_export(desc: "ModelInput", k: int, low: int = 0) -> dict:
+    """The S = 1 passes for tiles of k sites, computed on the host (pned_q3_plan_export)."""
+    n = C.c_int64(0)
+    check(lib().pned_q3_plan_export(C.byref(desc.c), int(k), int(low), None, 0, C.byref(n)))
+    buf = np.zeros(n.value, dtype=np.int64)
+    check(lib().pned_q3_plan_export(C.byref(desc.c), int(k), int(low), buf.ctypes.data_as(C.POINTER(C.c_int64)),
+                                    n.value, C.byref(n)))
+    it = iter(buf.tolist())
+    nsites, nr = next(it), next(it)
+    rterms = [dict(zip(("offset", "s1", "s2", "tab"), (next(it) for _ in range(4)))) for _ in range(nr)]
+    nonzero = [next(it) for _ in range(next(it))]
+    passes = []
+    for _ in range(next(it)):
+        kk, nout, nsub, ntab = (next(it) for _ in range(4))
+        ps = {"sites": [next(it) for _ in range(kk)], "outer": [next(it) for _ in range(nout)]}
+        ps["members"] = [dict(zip(("loff", "tab", "var", "first", "sh1", "sh2", "m1", "m2"),
+                                  (next(it) for _ in range(8)))) for _ in range(nsub)]
+        ps["tsrc"] = [next(it) for _ in range(ntab)]
+        passes.append(ps)
+    return {"n": nsites, "rterms": rterms, "nonzero": nonzero, "passes": passes}
+
+
 class Model:
     """A compiled model on the current device (pned_model_create)."""
 

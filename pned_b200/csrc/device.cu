@@ -1038,6 +1038,7 @@ int hv_partial_blocks(const pned_model *m, int R, int nblocks)
     if (const pned_model::XTileSet *xs = find_xtiles(m, R)) return int(xtile_rows(m, *xs, R, nblocks, false));
     if (!m->tprogs.empty() && R == 1 && m->use_tile) return int(m->tprogs.size()) * tile_grid(m, nblocks);
     if (const pned_model::TileSet *ts = find_rtiles(m, R)) return int(ts->progs.size()) * rtile_grid(m, nblocks);
+    if (const pned_model::Q3Set *qs = find_q3(m, R)) return int(qs->progs.size()) * q3_grid(m, *qs, nblocks);
     if (const pned_model::QTileSet *qs = find_qtiles(m, R)) return int(qs->progs.size()) * qtile_grid(m, *qs, nblocks);
     if (R == 1 && sector_segments_on(m)) return sector_grid(m, nblocks);
     return nblocks;
@@ -1057,6 +1058,7 @@ cudaError_t launch_hv(const pned_model *m, const HvArgs &a, int nblocks, cudaStr
         if (a.K == 4) return launch_rv<4>(m, *ts, a, nblocks, st);
     }
     if (a.slot_tables) return cudaErrorInvalidValue;
+    if (const pned_model::Q3Set *qs = find_q3(m, a.R)) return launch_q3(m, *qs, a, nblocks, st);
     if (const pned_model::QTileSet *qs = find_qtiles(m, a.R)) return launch_qtile(m, *qs, a, nblocks, st);
     if (a.R == 1 && sector_segments_on(m)) return launch_sector(m, sector_args(m, a), nblocks, st);
     switch (a.K) {
@@ -1079,7 +1081,8 @@ cudaError_t launch_hv_sums(const pned_model *m, const HvArgs &a, int nblocks, do
     const int kr = a.K * a.R;
     const bool staged = a.R == 1 && !m->tprogs.empty() && m->use_tile && !find_xtiles(m, 1) && tile_staged(m);
     HvArgs b = a;
-    const bool in = a.fin.done && kr == 1 && !staged && rows <= kFinishInKernel;
+    // the S = 1 kernel (its block size varies) leaves them to the finish kernels
+    const bool in = a.fin.done && kr == 1 && !staged && !find_q3(m, a.R) && rows <= kFinishInKernel;
     if (in_kernel) *in_kernel = in;
     if (in) {
         b.fin.base = a.partials;
@@ -1505,8 +1508,12 @@ extern "C" int pned_model_plan(const pned_model *m, int R, int *tile_passes, int
         states = kThreads * (1 << m->tile_jb);
     } else if (m->q > 2) {
         std::lock_guard<std::mutex> lock(const_cast<pned_model *>(m)->rtiles_mu);
+        auto i3 = m->q3.find(R);
         auto it = m->qtiles.find(R);
-        if (it != m->qtiles.end() && !it->second.progs.empty()) {
+        if (i3 != m->q3.end() && !i3->second.progs.empty()) {
+            passes = int(i3->second.progs.size());
+            states = i3->second.progs[0]->nt;
+        } else if (it != m->qtiles.end() && !it->second.progs.empty()) {
             passes = int(it->second.progs.size());
             states = it->second.progs[0]->nt;
         }
@@ -1616,7 +1623,7 @@ extern "C" int pned_ctx_create(pned_model *m, int R, size_t budget, pned_ctx **o
     // tiled kernels write one partial sum per block and pass
     if (R == 1 ? !m->plan1_set : !m->rtiles_set.count(R)) ensure_xtiles(m, R, false);
     if (R > 1 && !find_xtiles(m, R)) ensure_rtiles(m, R, false, nullptr);
-    ensure_qtiles(m, R);
+    if (!ensure_q3(m, R)) ensure_qtiles(m, R);
     // room for per-block sums, and for R = 1 for the per-tile sums of the dynamic tile
     // order: the current plan, or any plan of two passes with tiles of >= 2048 states
     size_t pslots = size_t(c->nblocks) * std::max(kTileMaxPasses, kQTileMaxPasses) * kMaxK * kMaxR;

@@ -62,6 +62,13 @@ struct pned_model {
         size_t smem = 0;
     };
     std::map<int, QTileSet> qtiles;
+    // S = 1 passes per R (guarded by rtiles_mu)
+    struct Q3Set {
+        std::vector<std::unique_ptr<pned::Q3Program>> progs;
+        int threads = 0;
+        size_t smem = 0;
+    };
+    std::map<int, Q3Set> q3;
     pned_tile_plan plan1{-1, -1, -1, -1, -1, -1, -1};   // single-vector plan parameters (-1: defaults)
     int tile_jb = 3;                        // j bits (rows per thread 2^jb) of the single-vector tiles
     int tile_bps = 2;                       // resident blocks per SM the single-vector tile kernel is built for
@@ -212,6 +219,11 @@ bool plan_default(const pned_tile_plan *p);
 int64_t xtile_rows(const pned_model *m, const pned_model::XTileSet &xs, int R, int nblocks, bool dynamic);
 cudaError_t launch_xtile(const pned_model *m, const pned_model::XTileSet &xs, const HvArgs &a, int nblocks,
                          cudaStream_t st);
+// The S = 1 kernel's passes for R (false or null: the kernel for any base runs), its grid and launch.
+bool ensure_q3(pned_model *m, int R);
+const pned_model::Q3Set *find_q3(const pned_model *m, int R);
+int q3_grid(const pned_model *m, const pned_model::Q3Set &qs, int nblocks);
+cudaError_t launch_q3(const pned_model *m, const pned_model::Q3Set &qs, const HvArgs &a, int nblocks, cudaStream_t st);
 bool ensure_qtiles(pned_model *m, int R);
 // Tile set of the mixed-radix tiled kernel for R (null: the flat kernel runs).
 const pned_model::QTileSet *find_qtiles(const pned_model *m, int R);

@@ -1132,6 +1132,96 @@ int plan_qtiles(const HostProgram &P, int k, int low, std::vector<QTilePass> &pa
     return PNED_OK;
 }
 
+int plan_q3(const HostProgram &P, int k, int low, std::vector<Q3Pass> &out)
+{
+    out.clear();
+    if (P.q != 3) return PNED_ENOTSUP;
+    for (const auto &d : P.rdelta)
+        if (std::abs(d.first) > 1 || std::abs(d.second) > 1) return PNED_ENOTSUP;
+    std::vector<QTilePass> passes;
+    const int rc = plan_qtiles(P, k, low, passes);
+    if (rc) return rc;
+    // a term by its bond's sites; a pass takes the terms of its bonds
+    for (const QTilePass &ps : passes) {
+        struct Term { int s1, s2, d1, d2, tab; };
+        std::vector<Term> terms;
+        for (const QTileTerm &t : ps.terms) {
+            const int s1 = ps.sites[t.ls1], s2 = ps.sites[t.ls2];
+            for (size_t i = 0; i < P.rterms.size(); ++i)   // the program's term (its table names it)
+                if (P.rterms[i].tab == t.tab) terms.push_back({s1, s2, P.rdelta[i].first, P.rdelta[i].second, int(t.tab)});
+        }
+        // offset outside J of a term (digit change and site), as a sortable key
+        auto key = [&](const Term &t, int a, int b) {
+            int64_t o = 0;
+            if (t.s1 != a && t.s1 != b && t.d1) o += int64_t(t.d1 + 2) << (2 * t.s1);
+            if (t.s2 != a && t.s2 != b && t.d2) o += int64_t(t.d2 + 2) << (2 * t.s2);
+            return o;
+        };
+        // J sites: the pair above the `low` lowest tile sites with the fewest row loads
+        int ja = ps.sites[k - 2], jb = ps.sites[k - 1], best = 1 << 20;
+        for (int x = low; x < k; ++x)
+            for (int y = x + 1; y < k; ++y) {
+                std::vector<int64_t> ks;
+                for (const Term &t : terms) ks.push_back(key(t, ps.sites[x], ps.sites[y]));
+                std::sort(ks.begin(), ks.end());
+                const int c = int(std::unique(ks.begin(), ks.end()) - ks.begin());
+                if (c < best) { best = c; ja = ps.sites[x]; jb = ps.sites[y]; }
+            }
+        Q3Pass q;
+        q.outer = ps.outer;
+        q.sites = {ja, jb};
+        for (int x : ps.sites)
+            if (x != ja && x != jb) q.sites.push_back(x);
+        int64_t lpw[17] = {1};
+        for (int i = 1; i <= k; ++i) lpw[i] = lpw[i - 1] * 3;
+        auto pos = [&](int x) { return int(std::find(q.sites.begin(), q.sites.end(), x) - q.sites.begin()); };
+        std::stable_sort(terms.begin(), terms.end(), [&](const Term &a, const Term &b) { return key(a, ja, jb) < key(b, ja, jb); });
+        for (size_t i = 0; i < terms.size(); ++i) {
+            const Term &t = terms[i];
+            const int p1 = pos(t.s1), p2 = pos(t.s2);
+            Q3Sub s{};
+            s.first = i == 0 || key(t, ja, jb) != key(terms[i - 1], ja, jb);
+            s.loff = int32_t((p1 > 1 ? t.d1 * lpw[p1] : 0) + (p2 > 1 ? t.d2 * lpw[p2] : 0));
+            const size_t tab = q.tsrc.size();
+            s.tab = uint16_t(tab);
+            q.tsrc.resize(tab + 9);
+            const bool j1 = p1 < 2, j2 = p2 < 2;
+            // digits (first index fastest): (d1, d2) outside J; (J digit, other digit); (ja, jb)
+            for (int e = 0; e < 9; ++e) {
+                const int u = e % 3, v = e / 3;
+                int g1 = u, g2 = v;   // digits of s1, s2
+                if (j1 && j2) {
+                    g1 = p1 == 0 ? u : v;
+                    g2 = p1 == 0 ? v : u;
+                } else if (j2) {
+                    g1 = v;
+                    g2 = u;
+                }
+                q.tsrc[tab + e] = t.tab + g1 + 3 * g2;
+            }
+            if (!j1 && !j2) {
+                s.var = 0;
+                s.sh1 = uint8_t(2 * (p1 - 2));
+                s.m1 = 1;
+                s.sh2 = uint8_t(2 * (p2 - 2));
+                s.m2 = 3;
+            } else if (j1 && j2) {
+                const int da = p1 == 0 ? t.d1 : t.d2, db = p1 == 0 ? t.d2 : t.d1;
+                const int code = (da + 1) + 3 * (db + 1);   // 4 is (0, 0), which is no term
+                s.var = uint8_t(7 + (code < 4 ? code : code - 1));
+            } else {
+                const int pj = j1 ? p1 : p2, dj = j1 ? t.d1 : t.d2, po = j1 ? p2 : p1;
+                s.var = uint8_t((pj == 0 ? 1 : 4) + dj + 1);
+                s.sh1 = uint8_t(2 * (po - 2));
+                s.m1 = 3;
+            }
+            q.subs.push_back(s);
+        }
+        out.push_back(q);
+    }
+    return PNED_OK;
+}
+
 }  // namespace pned
 
 // ---------------------------------------------------------------------------
@@ -1246,6 +1336,37 @@ extern "C" int pned_qtile_plan_export(const pned_model_desc *d, int k, int low, 
         for (int x : ps.outer) v.push_back(x);
         for (const QTileTerm &t : ps.terms)
             v.insert(v.end(), {int64_t(t.loff), int64_t(t.ls1), int64_t(t.ls2), int64_t(t.tab)});
+    }
+    *len = int64_t(v.size());
+    for (int64_t i = 0; i < std::min<int64_t>(cap, *len); ++i) out[i] = v[size_t(i)];
+    return PNED_OK;
+}
+
+// S = 1 passes of hv_q3.cu for tiles of k sites (the `low` lowest in every tile, none of
+// them a J site): the program's radix terms, then every pass.
+extern "C" int pned_q3_plan_export(const pned_model_desc *d, int k, int low, int64_t *out, int64_t cap, int64_t *len)
+{
+    using namespace pned;
+    if (!d || !len || (cap > 0 && !out)) return fail(PNED_EINVAL, "pned_q3_plan_export: bad arguments");
+    HostProgram P;
+    int rc = compile_program(d, P);
+    if (rc) return rc;
+    std::vector<Q3Pass> passes;
+    rc = P.sector ? PNED_ENOTSUP : plan_q3(P, k, low, passes);
+    if (rc) return fail(rc, "pned_q3_plan_export: no S = 1 passes for this model");
+    std::vector<int64_t> v{int64_t(P.n), int64_t(P.rterms.size())};
+    for (const RadixTerm &t : P.rterms) v.insert(v.end(), {t.offset, int64_t(t.s1), int64_t(t.s2), int64_t(t.tab)});
+    v.push_back(int64_t(P.table.size()));
+    for (const cd &z : P.table) v.push_back(z != cd(0, 0) ? 1 : 0);
+    v.push_back(int64_t(passes.size()));
+    for (const Q3Pass &q : passes) {
+        v.insert(v.end(), {int64_t(q.sites.size()), int64_t(q.outer.size()), int64_t(q.subs.size()), int64_t(q.tsrc.size())});
+        for (int x : q.sites) v.push_back(x);
+        for (int x : q.outer) v.push_back(x);
+        for (const Q3Sub &t : q.subs)
+            v.insert(v.end(), {int64_t(t.loff), int64_t(t.tab), int64_t(t.var), int64_t(t.first), int64_t(t.sh1),
+                               int64_t(t.sh2), int64_t(t.m1), int64_t(t.m2)});
+        for (int x : q.tsrc) v.push_back(x);
     }
     *len = int64_t(v.size());
     for (int64_t i = 0; i < std::min<int64_t>(cap, *len); ++i) out[i] = v[size_t(i)];

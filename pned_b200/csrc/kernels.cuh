@@ -78,6 +78,16 @@ struct TileProgram {
     TileTerm t[kMaxTerms];
 };
 
+// One pass of the S = 1 kernel (see Q3Sub).
+struct Q3Program {
+    int k, nt, vs, nouter, nsub, ntab, first, last;
+    int64_t ntiles;
+    uint32_t spow[8], rank[8];      // 3^site of local digit i, and its weight among the tile's sites
+    uint32_t opow[32];
+    Q3Sub s[kQ3MaxSubs];
+    double2 tab[kQ3MaxTab];
+};
+
 // One pass of the class-tiled kernel (see XSub): tiles of 256 * 8 elements --
 // `rc` = 2^lr of the R vectors times 2^(11 - lr) states.
 struct XTileProgram {

@@ -116,6 +116,26 @@ struct QTilePass {
     std::vector<QTileTerm> terms;
 };
 
+// S = 1 (base 3) pass of hv_q3.cu: a thread owns the 9 states of two J sites (local digits
+// 0 and 1).  A member's rows start loff slots away; its coefficient is
+// table[tab + digit(sh1) * m1 + digit(sh2) * m2 + J part], its J shift fixed by var:
+// 0 none; 1..3 (da = -1, 0, 1; the bond's other site outside J); 4..6 the same for db;
+// 7..14 both sites in J, (da, db) in order.
+struct Q3Sub {
+    int32_t loff;
+    uint16_t tab;
+    uint8_t var, first;      // first of its class: loads the rows
+    uint8_t sh1, sh2, m1, m2;
+};
+constexpr int kQ3MaxSubs = 160;
+constexpr int kQ3MaxTab = 512;
+struct Q3Pass {
+    std::vector<int> sites;   // tile sites: the J sites, then the others ascending
+    std::vector<int> outer;
+    std::vector<Q3Sub> subs;
+    std::vector<int> tsrc;    // table entry -> entry of the program's table (-1: zero)
+};
+
 struct HostProgram {
     int n = 0, q = 2;
     int64_t dim = 0;                     // basis size: q^n, or the sector size
@@ -165,6 +185,9 @@ struct HostProgram {
 // site set grown from the most connected uncovered bond (plus the `low`
 // lowest sites, kept in every tile for contiguous runs of states).
 int plan_qtiles(const HostProgram &P, int k, int low, std::vector<QTilePass> &passes);
+// The same passes (q == 3) as hv_q3.cu takes them; PNED_ENOTSUP for elements that move a
+// digit by two.
+int plan_q3(const HostProgram &P, int k, int low, std::vector<Q3Pass> &passes);
 int plan_tiles(const HostProgram &P, int tbits, int jb, int fixed, int window_bits, int max_passes,
                std::vector<HostProgram::TilePass> &out, int objective = 0);
 

@@ -379,3 +379,44 @@ def test_class_tiled_plan_matches_every_flip_term(n, R, field):
             assert src.min() >= 0 and src.max() < tabsize
             got.append((tuple(part.tolist()), tuple(src.tolist())))
     assert len(got) == len(r["xterms"]) and set(got) == want
+
+
+@pytest.mark.parametrize("L1,L2,k,low,field", [(3, 2, 5, 0, False), (3, 2, 6, 1, True), (2, 2, 4, 0, True), (3, 2, 7, 1, False)])
+def test_s1_members_match_every_radix_term(L1, L2, k, low, field):
+    """The S = 1 kernel's members, followed through the thread's nine J states, the row
+    offset, the J shift and the packed table, give for every state the partner state and
+    the table entry of the radix terms: each (state, term) whose element is nonzero once,
+    and nothing else with a nonzero element."""
+    cl = honeycomb(L1, L2)
+    cpl = CP.kitaev_heisenberg(0.2, -1.0, gamma=0.1 if field else 0.0)
+    X, skip, pt = P.build_xlocal(3, 1, cpl, field=CP.field_111(0.05) if field else None)
+    r = api.q3_plan_export(P.ModelInput(cl.n, 3, 1, cl.ipair, cl.ibond_type, X, skip, pt), k, low)
+    n, nz = r["n"], np.array(r["nonzero"])
+    s = np.unique(np.concatenate([[0, 3 ** n - 1], np.random.default_rng(k).integers(0, 3 ** n, 3000)]))
+    digit = lambda x, i: (x // 3 ** i) % 3  # noqa: E731
+    pairs = lambda part, ent: np.stack([s, part, ent], 1)[nz[ent] != 0]  # noqa: E731
+    want = [pairs(s + t["offset"], t["tab"] + digit(s, t["s1"]) + 3 * digit(s, t["s2"])) for t in r["rterms"]]
+    jd = [(-1, -1), (0, -1), (1, -1), (-1, 0), (1, 0), (-1, 1), (0, 1), (1, 1)]
+    got = []
+    for ps in r["passes"]:
+        sites, src = ps["sites"], np.array(ps["tsrc"])
+        assert sorted(sites + ps["outer"]) == list(range(n)) and len(sites) == k
+        loc = sum(digit(s, x) * 3 ** i for i, x in enumerate(sites))   # local slot
+        ja, jb, t9 = loc % 3, loc // 3 % 3, loc // 9 * 9
+        rest = sum(((loc // 3 ** (i + 2)) % 3) << (2 * i) for i in range(k - 2))
+        new = False
+        for m in ps["members"]:
+            new = new or m["first"]
+            assert new and m["loff"] % 9 == 0
+            v = m["var"]
+            da, db = (0, 0) if v == 0 else ((v - 2, 0) if v < 4 else ((0, v - 5) if v < 7 else jd[v - 7]))
+            jp = 0 if v == 0 else (ja if v < 4 else (jb if v < 7 else ja + 3 * jb))
+            ent = m["tab"] + ((rest >> m["sh1"]) & 3) * m["m1"] + ((rest >> m["sh2"]) & 3) * m["m2"] + jp
+            ok = (ja + da >= 0) & (ja + da <= 2) & (jb + db >= 0) & (jb + db <= 2)
+            row = np.clip(t9 + m["loff"], 0, 3 ** k - 9)
+            ploc = row + (ja + da) + 3 * (jb + db)
+            part = s + sum(((ploc // 3 ** i) % 3 - digit(s, x)) * 3 ** x for i, x in enumerate(sites))
+            got.append(pairs(part, src[ent])[ok[nz[src[ent]] != 0]])
+            assert np.all(nz[src[ent[~ok]]] == 0)   # rows that the J shift drops have zero elements
+    order = lambda x: x[np.lexsort(x.T)]  # noqa: E731
+    assert np.array_equal(order(np.concatenate(got)), order(np.concatenate(want)))
