@@ -1392,7 +1392,8 @@ extern "C" int pned_bisec(const double *alpha, const double *beta, int ndim, dou
         double a = E[k - 1];
         for (int it = 0; it < 100; ++it) {
             const double c = (a + b) / 2.0;
-            if (std::fabs(a - b) < epsabs) continue;
+            if (std::fabs(a - b) < epsabs) break;   // (nothing changes any more)
+            const double a0 = a, b0 = b;
             int numneg = 0, ipass = 0;
             double g = 1.0;
             for (int i = 1; i <= ndim; ++i) {
@@ -1410,6 +1411,9 @@ extern "C" int pned_bisec(const double *alpha, const double *beta, int ndim, dou
                 a = c;
                 for (int i = k; i <= std::min(numneg, ne); ++i) E[i - 1] = c;
             }
+            // the interval is down to neighbouring numbers: the reference's remaining
+            // iterations repeat this one (about half of its 100; 32 steps: 0.2 -> 0.1 ms)
+            if (a == a0 && b == b0) break;
         }
     }
     return PNED_OK;

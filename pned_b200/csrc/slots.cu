@@ -8,10 +8,10 @@
 // Per step (one CUDA graph per three steps, since buffer roles rotate P -> C -> W):
 //   slot_hv_kernel        W = pc P + hsc (H_r - shift) C  with per-slot tables and
 //                         diagonal; sums <v|hv>, ||W||^2, <g|W>, <g|v>
-//                         (4R sums: in its last block, or the finish kernels)
+//   finish                4R sums
 //   slot_residual_kernel  Lanczos slots: W <- W - Re(alpha) v, beta^2 = ||W - alpha v||^2;
-//                         eigenvector slots also accumulate x += c_k v
-//                         its last block: R sums, then slot_epilogue: per-slot alpha/beta/TPS coefficients and next scales
+//                         eigenvector slots also accumulate x += c_k v; its last block adds
+//                         the R sums and runs slot_epilogue: per-slot alpha/beta/TPS coefficients and next scales
 // Lanczos follows S_one_half/Hybrid_TPS_Lanczos.f90:48-163 (alpha from the H.v
 // product, beta through the complex alpha, update with the real alpha), TPS
 // follows S_one_half/Hybrid_TPS_TPS.f90:325-409 and eval_phys_val :83-111, the
