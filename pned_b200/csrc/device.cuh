@@ -33,6 +33,7 @@ struct pned_model {
     int n = 0, q = 2, nbond = 0;
     int64_t dim = 0;
     bool real_coef = true, real_diag = true;
+    bool table_varies = false;   // the table's values change after creation (slot batches)
     int ntab = 0, nterms = 0;
     std::unique_ptr<pned::XorProgram> xprog;
     std::unique_ptr<pned::RadixProgram> rprog;

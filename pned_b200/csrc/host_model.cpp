@@ -976,6 +976,7 @@ int plan_xtiles(const HostProgram &P, int sbits, int fixed, int max_passes, std:
                 if (tab > 0xffff) return PNED_ENOTSUP;
                 const int M = var == kXGeneric ? 7 : kXVarM[var], nj = __builtin_popcount(unsigned(M));
                 ps.tsrc.resize(tab + (size_t(1) << (width + nj)), -1);
+                bool real = true;
                 for (int c = 0; c < (1 << int(pos.size())); ++c) {
                     uint32_t x = 0;
                     int idx = 0;
@@ -990,10 +991,11 @@ int plan_xtiles(const HostProgram &P, int sbits, int fixed, int max_passes, std:
                             ++i2;
                         }
                         ps.tsrc[tab + (size_t(h) << nj) + u] = t.tab + id;
+                        if (P.table[t.tab + id].imag() != 0) real = false;
                     }
                 }
                 s.pack = uint32_t(var + 16 * d + (first ? 128 : 0)) | uint32_t(width ? 32 - width : 0) << 8 |
-                         uint32_t(tab) << 16;
+                         (real ? kXReal : 0u) | uint32_t(tab) << 16;
                 first = false;
                 if (!g.in) ++ps.nout;
                 ps.subs.push_back(s);

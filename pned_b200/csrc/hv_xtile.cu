@@ -56,32 +56,40 @@ namespace pned {
 #define PNED_XL2(L) L(0) L(1)
 #define PNED_XL4(L) L(0) L(1) L(2) L(3)
 #define PNED_XL8(L) L(0) L(1) L(2) L(3) L(4) L(5) L(6) L(7)
-#define PNED_XBODY(F, L)                                                                              \
-    "{\n.reg .f64 x<8>, y<8>, z<8>;\n.reg .u32 t, p;\n"                                               \
-    "TS: .branchtargets V0, V1, V2, V3, V4, V5, V6, V7, V8, V9, V10, V11, V12, V13, V14;\n"           \
-    "brx.idx.uni %35, TS;\n"                                                                         \
-    "V0:\n" PNED_XPTR(0) PNED_XL1(L) PNED_XROWS(F, 0, 0, 0, 0, 0, 0, 0, 0, 0, 1, 2, 3, 4, 5, 6, 7)    \
-    "V1:\n" PNED_XPTR(1) PNED_XL2(L) PNED_XROWS(F, 0, 1, 0, 1, 0, 1, 0, 1, 0, 1, 2, 3, 4, 5, 6, 7)    \
-    "V2:\n" PNED_XPTR(1) PNED_XL2(L) PNED_XROWS(F, 0, 0, 1, 1, 0, 0, 1, 1, 0, 1, 2, 3, 4, 5, 6, 7)    \
-    "V3:\n" PNED_XPTR(1) PNED_XL2(L) PNED_XROWS(F, 0, 0, 0, 0, 1, 1, 1, 1, 0, 1, 2, 3, 4, 5, 6, 7)    \
-    "V4:\n" PNED_XPTR(2) PNED_XL4(L) PNED_XROWS(F, 0, 1, 2, 3, 0, 1, 2, 3, 0, 1, 2, 3, 4, 5, 6, 7)    \
-    "V5:\n" PNED_XPTR(2) PNED_XL4(L) PNED_XROWS(F, 0, 1, 0, 1, 2, 3, 2, 3, 0, 1, 2, 3, 4, 5, 6, 7)    \
-    "V6:\n" PNED_XPTR(2) PNED_XL4(L) PNED_XROWS(F, 0, 0, 1, 1, 2, 2, 3, 3, 0, 1, 2, 3, 4, 5, 6, 7)    \
-    "V7:\nV14:\n" PNED_XPTR(3) PNED_XL8(L) PNED_XROWS(F, 0, 1, 2, 3, 4, 5, 6, 7, 0, 1, 2, 3, 4, 5, 6, 7) \
-    "V8:\n" PNED_XPTR(1) PNED_XL2(L) PNED_XROWS(F, 0, 1, 0, 1, 0, 1, 0, 1, 1, 0, 3, 2, 5, 4, 7, 6)    \
-    "V9:\n" PNED_XPTR(1) PNED_XL2(L) PNED_XROWS(F, 0, 0, 1, 1, 0, 0, 1, 1, 2, 3, 0, 1, 6, 7, 4, 5)    \
-    "V10:\n" PNED_XPTR(1) PNED_XL2(L) PNED_XROWS(F, 0, 0, 0, 0, 1, 1, 1, 1, 4, 5, 6, 7, 0, 1, 2, 3)   \
-    "V11:\n" PNED_XPTR(2) PNED_XL4(L) PNED_XROWS(F, 0, 1, 2, 3, 0, 1, 2, 3, 3, 2, 1, 0, 7, 6, 5, 4)   \
-    "V12:\n" PNED_XPTR(2) PNED_XL4(L) PNED_XROWS(F, 0, 1, 0, 1, 2, 3, 2, 3, 5, 4, 7, 6, 1, 0, 3, 2)   \
-    "V13:\n" PNED_XPTR(2) PNED_XL4(L) PNED_XROWS(F, 0, 0, 1, 1, 2, 2, 3, 3, 6, 7, 4, 5, 2, 3, 0, 1)   \
-    "DONE:\n}\n"
+// all variants with labels P0 .. P14, products F and table reads L
+#define PNED_XALL(P, F, L) \
+    P "0:\n" PNED_XPTR(0) PNED_XL1(L) PNED_XROWS(F, 0, 0, 0, 0, 0, 0, 0, 0, 0, 1, 2, 3, 4, 5, 6, 7)    \
+    P "1:\n" PNED_XPTR(1) PNED_XL2(L) PNED_XROWS(F, 0, 1, 0, 1, 0, 1, 0, 1, 0, 1, 2, 3, 4, 5, 6, 7)    \
+    P "2:\n" PNED_XPTR(1) PNED_XL2(L) PNED_XROWS(F, 0, 0, 1, 1, 0, 0, 1, 1, 0, 1, 2, 3, 4, 5, 6, 7)    \
+    P "3:\n" PNED_XPTR(1) PNED_XL2(L) PNED_XROWS(F, 0, 0, 0, 0, 1, 1, 1, 1, 0, 1, 2, 3, 4, 5, 6, 7)    \
+    P "4:\n" PNED_XPTR(2) PNED_XL4(L) PNED_XROWS(F, 0, 1, 2, 3, 0, 1, 2, 3, 0, 1, 2, 3, 4, 5, 6, 7)    \
+    P "5:\n" PNED_XPTR(2) PNED_XL4(L) PNED_XROWS(F, 0, 1, 0, 1, 2, 3, 2, 3, 0, 1, 2, 3, 4, 5, 6, 7)    \
+    P "6:\n" PNED_XPTR(2) PNED_XL4(L) PNED_XROWS(F, 0, 0, 1, 1, 2, 2, 3, 3, 0, 1, 2, 3, 4, 5, 6, 7)    \
+    P "7:\n" P "14:\n" PNED_XPTR(3) PNED_XL8(L) PNED_XROWS(F, 0, 1, 2, 3, 4, 5, 6, 7, 0, 1, 2, 3, 4, 5, 6, 7) \
+    P "8:\n" PNED_XPTR(1) PNED_XL2(L) PNED_XROWS(F, 0, 1, 0, 1, 0, 1, 0, 1, 1, 0, 3, 2, 5, 4, 7, 6)    \
+    P "9:\n" PNED_XPTR(1) PNED_XL2(L) PNED_XROWS(F, 0, 0, 1, 1, 0, 0, 1, 1, 2, 3, 0, 1, 6, 7, 4, 5)    \
+    P "10:\n" PNED_XPTR(1) PNED_XL2(L) PNED_XROWS(F, 0, 0, 0, 0, 1, 1, 1, 1, 4, 5, 6, 7, 0, 1, 2, 3)   \
+    P "11:\n" PNED_XPTR(2) PNED_XL4(L) PNED_XROWS(F, 0, 1, 2, 3, 0, 1, 2, 3, 3, 2, 1, 0, 7, 6, 5, 4)   \
+    P "12:\n" PNED_XPTR(2) PNED_XL4(L) PNED_XROWS(F, 0, 1, 0, 1, 2, 3, 2, 3, 5, 4, 7, 6, 1, 0, 3, 2)   \
+    P "13:\n" PNED_XPTR(2) PNED_XL4(L) PNED_XROWS(F, 0, 0, 1, 1, 2, 2, 3, 3, 6, 7, 4, 5, 2, 3, 0, 1)
+#define PNED_XREGS "{\n.reg .f64 x<8>, y<8>, z<8>;\n.reg .u32 t, p;\n"
+#define PNED_XTARGETS(P) \
+    P "0, " P "1, " P "2, " P "3, " P "4, " P "5, " P "6, " P "7, " P "8, " P "9, " P "10, " P "11, " P "12, " P "13, " P "14"
+// real coefficients only, or complex ones with the real members' variants behind them (16 on)
+#define PNED_XBODY_R                                                                            \
+    PNED_XREGS "TS: .branchtargets " PNED_XTARGETS("V") ";\nbrx.idx.uni %35, TS;\n"             \
+    PNED_XALL("V", PNED_XFR, PNED_XLR) "DONE:\n}\n"
+#define PNED_XBODY_C                                                                                              \
+    PNED_XREGS "TS: .branchtargets " PNED_XTARGETS("V") ", V14, " PNED_XTARGETS("U") ";\nbrx.idx.uni %35, TS;\n"   \
+    PNED_XALL("V", PNED_XFC, PNED_XLC) PNED_XALL("U", PNED_XFR, PNED_XLR) "DONE:\n}\n"
 
 template <bool RC>
 __device__ __forceinline__ void x_member(const uint4 &S, uint32_t base, uint32_t tab, uint32_t ts,
                                          const double2 (&w)[kXSPT], double2 (&acc)[kXSPT])
 {
     static_assert(kXSPT == 8, "the variants below are written for 8 states a thread");
-    const uint32_t h = ((base & S.x) * S.y) >> ((S.w >> 8) & 31u), ct = tab + (S.w >> 16) * ts, var = S.w & 15u;
+    const uint32_t h = ((base & S.x) * S.y) >> ((S.w >> 8) & 31u), ct = tab + (S.w >> 16) * ts;
+    const uint32_t var = (S.w & 15u) | (RC ? 0u : (S.w >> 9) & 16u);   // kXReal: the real variants
 #define PNED_XOPS                                                                                                        \
     "+d"(acc[0].x), "+d"(acc[0].y), "+d"(acc[1].x), "+d"(acc[1].y), "+d"(acc[2].x), "+d"(acc[2].y), "+d"(acc[3].x),      \
         "+d"(acc[3].y), "+d"(acc[4].x), "+d"(acc[4].y), "+d"(acc[5].x), "+d"(acc[5].y), "+d"(acc[6].x), "+d"(acc[6].y),  \
@@ -90,8 +98,8 @@ __device__ __forceinline__ void x_member(const uint4 &S, uint32_t base, uint32_t
           "d"(w[4].x), "d"(w[4].y), "d"(w[5].x), "d"(w[5].y), "d"(w[6].x), "d"(w[6].y), "d"(w[7].x), "d"(w[7].y),        \
           "r"(ct), "r"(h), "r"(ts), "r"(var)                                                                             \
         : "memory"
-    if (RC) asm volatile(PNED_XBODY(PNED_XFR, PNED_XLR) : PNED_XOPS);
-    else asm volatile(PNED_XBODY(PNED_XFC, PNED_XLC) : PNED_XOPS);
+    if (RC) asm volatile(PNED_XBODY_R : PNED_XOPS);
+    else asm volatile(PNED_XBODY_C : PNED_XOPS);
 #undef PNED_XOPS
 }
 
@@ -106,7 +114,7 @@ __device__ __forceinline__ void x_member(const uint4 &S, uint32_t base, uint32_t
 // SM: fp64 pipe 28 %, issue 46 %.  Hence the classes (60 masks become 40 row reads at
 // N = 24), the perfect hash (3 instructions for a coefficient index), members as one
 // 16-byte constant read fetched ahead, and the indexed jump.  Measured H.V against the
-// multi-vector kernel: N = 24, R = 16 with a field 18.6 -> 13.2 ms, R = 12 without
+// multi-vector kernel: N = 24, R = 16 with a field 18.6 -> 13.0 ms, R = 12 without
 // 12.0 -> 8.3 ms, N = 22, R = 2 0.69 -> 0.49 ms, N = 26, R = 4 21.5 -> 14.3 ms.
 // Measured and dropped: a second class in flight through cp.async (15.1 against 14.8 ms:
 // the address arithmetic costs more than the latency it hides).
@@ -345,7 +353,7 @@ bool ensure_xtiles(pned_model *m, int R, bool slot_tables)
         for (int k = 0; k < T->nouter; ++k) T->outer[k] = uint8_t(t.outer[k]);
         for (size_t i = 0; i < t.subs.size(); ++i) {
             const XSub &q = t.subs[i];
-            T->s[i] = make_uint4(q.dmask, q.mul, q.mask, q.pack);
+            T->s[i] = make_uint4(q.dmask, q.mul, q.mask, m->table_varies ? q.pack & ~kXReal : q.pack);
         }
         xs.groups += t.groups;
         xs.progs.push_back(std::move(T));

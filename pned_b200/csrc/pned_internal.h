@@ -88,8 +88,9 @@ constexpr int kTileMaxGroups = 64;    // partner tiles per pass
 struct XSub {
     uint32_t dmask, mul;
     uint32_t mask;     // the class's partner rows -- in-tile: local row xor; out-of-tile: global xor (no J bits)
-    uint32_t pack;     // variant + 16 * (J bits flipped) + 128 * (first of its class) + sh << 8 + tab << 16
+    uint32_t pack;     // variant + 16 * (J bits flipped) + 128 * (first of its class) + sh << 8 + kXReal + tab << 16
 };
+constexpr uint32_t kXReal = 1u << 13;   // every value of the member is real: half the products
 // Variants, each with fixed J bits flipped (D) and fixed J dependencies (M): the ones
 // that two-site flips on lattices with few common neighbours need.  Any other member is
 // its own class under kXGeneric, its rows loaded with D applied and its table holding

@@ -650,6 +650,7 @@ extern "C" int pned_slots_create(const pned_model_desc *structure, int R, int ma
         m.hp = S->hp;
         m.device = S->device; m.n = S->n; m.q = 2; m.nbond = S->nbond; m.dim = S->dim;
         m.real_coef = false; m.real_diag = true;
+        m.table_varies = true;
         m.ntab = S->ntab; m.nterms = S->xprog->nterms; m.nsm = S->nsm;
         m.d_table = S->table; m.d_diag = S->diag;
         if (R == 1) {
