@@ -344,7 +344,7 @@ __global__ void __launch_bounds__(kThreads, BPS)
     }
     // static order: the block's sums over its tiles (same reduction order)
     if (!ctr) tile_sums_store<K>(red, s_red, a.partials + size_t(blockIdx.x) * K);
-    if (prog.last) hv_finish(a);
+    if (prog.last) hv_finish(a, smem);
 }
 
 // Tiled multi-vector H.V (R > 1 interleaved vectors, S = 1/2 full basis), one
@@ -545,7 +545,7 @@ __global__ void __launch_bounds__(kThreads, 2) hv_tile_rv_kernel(const __grid_co
         chunk = s_next;
     }
     if (!ctr) block_reduce_store<K, VPT, true>(red, G, VPT, R, a.partials);
-    if (prog.last) hv_finish(a);
+    if (prog.last) hv_finish(a, smem);
 }
 
 // Mixed-radix (q > 2) variant: partner = s + offset, coefficient indexed by
@@ -1081,8 +1081,9 @@ cudaError_t launch_hv_sums(const pned_model *m, const HvArgs &a, int nblocks, do
     const int kr = a.K * a.R;
     const bool staged = a.R == 1 && !m->tprogs.empty() && m->use_tile && !find_xtiles(m, 1) && tile_staged(m);
     HvArgs b = a;
-    // the S = 1 kernel (its block size varies) leaves them to the finish kernels
-    const bool in = a.fin.done && kr == 1 && !staged && !find_q3(m, a.R) && rows <= kFinishInKernel;
+    // the S = 1 kernel (its block size varies) and the sector's segment kernel (at its register
+    // limit: 1 % slower with the sums in it, N = 28) leave them to the finish kernels
+    const bool in = a.fin.done && kr == 1 && !staged && !find_q3(m, a.R) && !sector_segments_on(m) && rows <= kFinishInKernel;
     if (in_kernel) *in_kernel = in;
     if (in) {
         b.fin.base = a.partials;

@@ -123,7 +123,6 @@ __global__ void __launch_bounds__(kThreads, 4)
         }
     }
     block_reduce_store<K, 1>(red, 1, 1, 1, a.partials);
-    hv_finish(a);
 }
 
 // Shared memory of the segment kernel: the table and one partner-segment
