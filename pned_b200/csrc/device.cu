@@ -1553,18 +1553,13 @@ extern "C" int pned_model_set_plan(pned_model *m, int R, const pned_tile_plan *p
         m->plan1_set = plan != nullptr;
         m->carveout = m->plan1.l1_carveout != 0;
         build_tile_programs(m);
-        if (plan) clear_xtiles(m, 1);
-        else ensure_xtiles(m, 1, false);
+        switch_xtiles(m, 1, !plan);
+        ensure_xtiles(m, 1, false);
         return PNED_OK;
     }
     if (plan) m->carveout = plan->l1_carveout != 0;
-    if (plan_default(plan)) {   // the class-tiled passes, where they run
-        m->rtiles_set.erase(R);
-        if (ensure_xtiles(m, R, false)) return PNED_OK;
-    } else {
-        m->rtiles_set.insert(R);
-        clear_xtiles(m, R);
-    }
+    switch_xtiles(m, R, plan_default(plan));   // the class-tiled passes, where they run
+    if (ensure_xtiles(m, R, false)) return PNED_OK;
     const pned_tile_plan def{-1, -1, -1, -1, -1, -1, -1, -1, -1};
     ensure_rtiles(m, R, false, plan ? plan : &def);
     return PNED_OK;
@@ -1622,8 +1617,7 @@ extern "C" int pned_ctx_create(pned_model *m, int R, size_t budget, pned_ctx **o
     if (e != cudaSuccess) return cuda_fail(e, "cudaStreamCreate");
     c->stream = c->own_stream;
     // tiled kernels write one partial sum per block and pass
-    if (R == 1 ? !m->plan1_set : !m->rtiles_set.count(R)) ensure_xtiles(m, R, false);
-    if (R > 1 && !find_xtiles(m, R)) ensure_rtiles(m, R, false, nullptr);
+    if (!ensure_xtiles(m, R, false) && R > 1) ensure_rtiles(m, R, false, nullptr);
     if (!ensure_q3(m, R)) ensure_qtiles(m, R);
     // room for per-block sums, and for R = 1 for the per-tile sums of the dynamic tile
     // order: the current plan, or any plan of two passes with tiles of >= 2048 states

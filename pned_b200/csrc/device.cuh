@@ -6,7 +6,6 @@
 #include <map>
 #include <memory>
 #include <mutex>
-#include <set>
 #include <vector>
 
 #include "kernels.cuh"
@@ -47,15 +46,18 @@ struct pned_model {
     };
     std::map<int, TileSet> rtiles;
     std::mutex rtiles_mu;
-    // class-tiled passes per R (q == 2, full basis; guarded by rtiles_mu): groups of 2^lr vectors
+    // class-tiled passes per R (q == 2, full basis; guarded by rtiles_mu): groups of 2^lr vectors.
+    // Built once and kept until the model goes: the graph of a running session holds
+    // the address of `mem` in its kernel parameters, so an explicit plan only sets `off`.
     struct XTileSet {
         std::vector<std::unique_ptr<pned::XTileProgram>> progs;
         int lr = 0;
         int groups = 0;   // partner tiles over all passes
+        bool built = false;   // planned (progs empty: no class-tiled plan)
+        bool off = false;     // an explicit plan takes its place
         pned::DevBuf mem; // the passes' table sources
     };
     std::map<int, XTileSet> xtiles;
-    std::set<int> rtiles_set;   // R > 1 with an explicit plan for the multi-vector kernel
     // tiled mixed-radix passes per R (q > 2, full basis; guarded by rtiles_mu)
     struct QTileSet {
         std::vector<std::unique_ptr<pned::QTileProgram>> progs;
@@ -210,11 +212,11 @@ bool ensure_rtiles(pned_model *m, int R, bool slot_tables, const pned_tile_plan 
 // Shared memory of the tiled multi-vector kernel for R vectors.
 size_t rtile_smem(const pned_model *m, int R, bool slot_tables);
 // Class-tiled passes for R vectors (S = 1/2, n >= 12), once per model and R; false:
-// another kernel runs.  The set for R (null: none; clear_xtiles: an explicit plan takes
-// its place), the partial-sum rows a call writes, and all its passes.
+// another kernel runs.  The set for R (null: none, or switched off because an explicit
+// plan takes its place), the partial-sum rows a call writes, and all its passes.
 bool ensure_xtiles(pned_model *m, int R, bool slot_tables);
 const pned_model::XTileSet *find_xtiles(const pned_model *m, int R);
-void clear_xtiles(pned_model *m, int R);
+void switch_xtiles(pned_model *m, int R, bool on);
 // No plan, or one whose every field asks for the default.
 bool plan_default(const pned_tile_plan *p);
 int64_t xtile_rows(const pned_model *m, const pned_model::XTileSet &xs, int R, int nblocks, bool dynamic);

@@ -303,7 +303,7 @@ const pned_model::XTileSet *find_xtiles(const pned_model *m, int R)
 {
     std::lock_guard<std::mutex> lock(const_cast<pned_model *>(m)->rtiles_mu);
     auto it = m->xtiles.find(R);
-    if (it == m->xtiles.end() || it->second.progs.empty()) return nullptr;
+    if (it == m->xtiles.end() || it->second.off || it->second.progs.empty()) return nullptr;
     return &it->second;
 }
 
@@ -327,8 +327,9 @@ bool ensure_xtiles(pned_model *m, int R, bool slot_tables)
     // another order may return -x where a caller had x.
     if (R == 1 && (m->real_coef || hp.n < kTileBigSites)) return false;
     std::lock_guard<std::mutex> lock(m->rtiles_mu);
-    if (m->xtiles.count(R)) return !m->xtiles[R].progs.empty();
     pned_model::XTileSet &xs = m->xtiles[R];
+    if (xs.off || xs.built) return !xs.off && !xs.progs.empty();
+    xs.built = true;
     std::vector<XTilePass> ps;
     if (plan_xtiles_for(hp, R, xs.lr, ps) != PNED_OK) return false;
     std::vector<uint16_t> tsrc;   // of all passes
@@ -369,10 +370,10 @@ bool ensure_xtiles(pned_model *m, int R, bool slot_tables)
     return true;
 }
 
-void clear_xtiles(pned_model *m, int R)
+void switch_xtiles(pned_model *m, int R, bool on)
 {
     std::lock_guard<std::mutex> lock(m->rtiles_mu);
-    m->xtiles.erase(R);
+    m->xtiles[R].off = !on;
 }
 
 static int xtile_grid(const pned_model *m, const pned_model::XTileSet &xs, int R, int nblocks)

@@ -862,13 +862,10 @@ extern "C" int pned_slots_set_plan(pned_slots *S, const pned_tile_plan *plan)
         build_tile_programs(&S->tm);
         S->tile = S->tm.use_tile;
     }
-    if (plan_default(plan)) {
-        if (ensure_xtiles(&S->tm, S->R, S->R > 1)) {
-            S->tile = true;
-            return PNED_OK;
-        }
-    } else {
-        clear_xtiles(&S->tm, S->R);
+    switch_xtiles(&S->tm, S->R, plan_default(plan));
+    if (ensure_xtiles(&S->tm, S->R, S->R > 1)) {
+        S->tile = true;
+        return PNED_OK;
     }
     if (S->R > 1) S->tile = ensure_rtiles(&S->tm, S->R, true, plan ? plan : &def);
     return PNED_OK;

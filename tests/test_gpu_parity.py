@@ -802,3 +802,36 @@ def test_class_tiled_and_in_kernel_sums_parity(n, R, field):
     for r in (0, R - 1):
         ref = om.lanczos(np.ascontiguousarray(V[:, r]), 8)
         assert rel(out["alpha"][:, r], ref["alpha"]) <= 1e-10 and rel(out["beta"][:, r], ref["beta"]) <= 1e-10
+
+
+@pytest.mark.parametrize("kind", ["lanczos", "tps"])
+def test_session_steps_on_after_a_plan_change(kind):
+    """A session whose captured steps run the class-tiled kernel steps on unharmed when the
+    model is given an explicit plan and its default back: the captured steps keep the table
+    sources that they were captured with, and the coefficients stay the uninterrupted
+    session's (10 steps of rounding apart: 1e-10, as against the oracle)."""
+    n, R, L = 14, 16, 28.0
+    X, skip, pt = P.build_xlocal(2, 0, KHGH, field=FIELD)
+    if kind == "tps":
+        X, _ = P.tps_transform(2, 0, n - 1, X, L=L)
+    ipair = np.array([[i + 1, i + 2] for i in range(n - 1)], dtype=np.int32).reshape(-1)
+    gm = P.Model(n, 2, 0, ipair, np.array([1 + i % 3 for i in range(n - 1)], dtype=np.int32), X, skip, pt)
+    v = O.gaussian(5, gm.dim, R).reshape(gm.dim, R)
+    v = np.ascontiguousarray(v / np.linalg.norm(v, axis=0)).reshape(-1)
+    runs = []
+    for change in (False, True):
+        ctx = P.Context(gm, R=R)
+        assert gm.plan(R)["tile_states"] == 256   # 2048 elements in groups of 8 vectors
+        ctx.session_begin(kind, v, 25, L=L)
+        ctx.session_step(7)                         # one step, then two replays of three
+        if change:
+            assert gm.set_plan(R, 0, 6, 2)["tile_states"] == 128
+        ctx.session_step(8)
+        if change:
+            assert gm.set_plan(R)["tile_states"] == 256
+        ctx.session_step(5)
+        runs.append(ctx.session_read())
+        ctx.session_end()
+        ctx.close()
+    for key in ("alpha", "beta"):
+        assert rel(runs[1][key], runs[0][key]) <= 1e-10
