@@ -1029,6 +1029,8 @@ extern "C" int pned_session_load(pned_ctx *c, const char *path, int max_steps)
     ok = ck_get(f, scal.data(), sizeof(double) * scal.size()) && ck_get(f, a.data(), sizeof(double) * nh) &&
          ck_get(f, b.data(), sizeof(double) * nh) && ck_get(f, cf.data(), sizeof(double) * cf.size());
     cudaError_t e = cudaSuccess;
+    // the ones are the context's own: files hold whatever their context had there
+    std::fill_n(scal.begin() + size_t(kSlotOne) * kMaxR, kMaxR, 1.0);
     if (ok) {
         e = cudaMemcpy(c->scal, scal.data(), sizeof(double) * scal.size(), cudaMemcpyHostToDevice);
         if (e == cudaSuccess && nh) e = cudaMemcpy(S.d_alpha, a.data(), sizeof(double) * nh, cudaMemcpyHostToDevice);

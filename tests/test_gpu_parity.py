@@ -835,3 +835,37 @@ def test_session_steps_on_after_a_plan_change(kind):
         ctx.close()
     for key in ("alpha", "beta"):
         assert rel(runs[1][key], runs[0][key]) <= 1e-10
+
+
+@pytest.mark.parametrize("junk", [0.0, float("nan")])
+def test_checkpoint_leaves_the_plain_products_scale_alone(junk, tmp_path):
+    """H.v and CG in a context that loaded a checkpoint: a file whose slot of ones holds
+    something else (files of contexts that had made no plain product yet) gives the same
+    bits as a context that loaded none."""
+    cl = honeycomb(2, 2)
+    gm, _ = models(cl, 2, 0, KH)
+    v = O.gaussian(3, gm.dim)
+    v /= np.linalg.norm(v)
+    a = P.Context(gm, R=1)
+    a.session_begin("lanczos", v, 8)
+    a.session_step(4)
+    path = str(tmp_path / "session.ckpt")
+    a.session_save(path)
+    a.session_end()
+    raw = bytearray(open(path, "rb").read())
+    # sections with 8-byte lengths: header (10 int32), dim, L, 2 counters, then the scalars, ones first
+    at = (8 + 40) + (8 + 8) + (8 + 8) + (8 + 8) + 8
+    assert np.all(np.frombuffer(raw, np.float64, 16, at) == 1.0)
+    raw[at:at + 128] = np.full(16, junk).tobytes()
+    open(path, "wb").write(raw)
+    out = []
+    for load in (False, True):
+        c = P.Context(gm, R=1)
+        if load:
+            c.session_load(path, 8)
+            c.session_end()
+        w = np.zeros_like(v)
+        pr = c.p_mltply_v3(v, w)
+        out.append((w, pr, c.cg(-5.0, v, inv_max=2, cg_max=20)[0]))
+    for x, y in zip(*out):
+        assert np.array_equal(x, y)
