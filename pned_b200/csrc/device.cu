@@ -1637,16 +1637,19 @@ extern "C" int pned_ctx_create(pned_model *m, int R, size_t budget, pned_ctx **o
     e = cudaMalloc(&c->partials, pbytes);
     if (e == cudaSuccess) e = cudaMalloc(&c->tile_ctr, sizeof(uint32_t) * kTileCounters);
     if (e == cudaSuccess) e = cudaMalloc(&c->fin_ctr, sizeof(uint32_t) * (1 + kTileCounters));
-    if (e == cudaSuccess) e = cudaMemset(c->fin_ctr, 0, sizeof(uint32_t) * (1 + kTileCounters));
     if (e == cudaSuccess) e = cudaMalloc(&c->sums, sizeof(double2) * kMaxK * kMaxR * 4);
     if (e == cudaSuccess) e = cudaMalloc(&c->scal, sizeof(double) * kScalSlots * kMaxR);
     if (e == cudaSuccess) e = cudaMallocHost(&c->h_sums, sizeof(double2) * (kMaxK * kMaxR * 4 + 1));
     if (e == cudaSuccess) e = cudaMalloc(&c->flag, sizeof(int) * 4);
-    if (e == cudaSuccess) e = cudaMemset(c->flag, 0, sizeof(int) * 4);
-    if (e == cudaSuccess) {   // the scale of plain products: ones, never written again
-        const std::vector<double> ones(kMaxR, 1.0);
-        e = cudaMemcpy(slot(c.get(), kSlotOne), ones.data(), sizeof(double) * kMaxR, cudaMemcpyHostToDevice);
-    }
+    // Zeroed counters and flag, and the scale of plain products (ones, never written again).
+    // On the context's stream and waited for: its stream does not wait for the legacy one,
+    // where a memset or a copy from pageable memory may still run when the call returns.
+    const std::vector<double> ones(kMaxR, 1.0);
+    if (e == cudaSuccess) e = cudaMemsetAsync(c->fin_ctr, 0, sizeof(uint32_t) * (1 + kTileCounters), c->stream);
+    if (e == cudaSuccess) e = cudaMemsetAsync(c->flag, 0, sizeof(int) * 4, c->stream);
+    if (e == cudaSuccess)
+        e = cudaMemcpyAsync(slot(c.get(), kSlotOne), ones.data(), sizeof(double) * kMaxR, cudaMemcpyHostToDevice, c->stream);
+    if (e == cudaSuccess) e = cudaStreamSynchronize(c->stream);
     if (e != cudaSuccess) {
         pned_ctx_destroy(c.release());
         return cuda_fail(e, "pned_ctx_create: scratch");

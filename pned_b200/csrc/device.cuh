@@ -21,7 +21,9 @@ struct DevBuf {
     bool upload(const void *src, size_t bytes)
     {
         if (cudaMalloc(&p, bytes ? bytes : 1) != cudaSuccess) { p = nullptr; cudaGetLastError(); return false; }
-        return cudaMemcpy(p, src, bytes, cudaMemcpyHostToDevice) == cudaSuccess;
+        // waited for: kernels on streams that do not wait for the legacy one read it next
+        return cudaMemcpyAsync(p, src, bytes, cudaMemcpyHostToDevice, cudaStreamPerThread) == cudaSuccess &&
+               cudaStreamSynchronize(cudaStreamPerThread) == cudaSuccess;
     }
 };
 }  // namespace pned

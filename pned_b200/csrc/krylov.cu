@@ -1031,13 +1031,13 @@ extern "C" int pned_session_load(pned_ctx *c, const char *path, int max_steps)
     cudaError_t e = cudaSuccess;
     // the ones are the context's own: files hold whatever their context had there
     std::fill_n(scal.begin() + size_t(kSlotOne) * kMaxR, kMaxR, 1.0);
-    if (ok) {
-        e = cudaMemcpy(c->scal, scal.data(), sizeof(double) * scal.size(), cudaMemcpyHostToDevice);
-        if (e == cudaSuccess && nh) e = cudaMemcpy(S.d_alpha, a.data(), sizeof(double) * nh, cudaMemcpyHostToDevice);
-        if (e == cudaSuccess && nh) e = cudaMemcpy(S.d_beta, b.data(), sizeof(double) * nh, cudaMemcpyHostToDevice);
+    if (ok) {   // on the session's stream, which the vectors' copies below wait for
+        e = cudaMemcpyAsync(c->scal, scal.data(), sizeof(double) * scal.size(), cudaMemcpyHostToDevice, c->stream);
+        if (e == cudaSuccess && nh) e = cudaMemcpyAsync(S.d_alpha, a.data(), sizeof(double) * nh, cudaMemcpyHostToDevice, c->stream);
+        if (e == cudaSuccess && nh) e = cudaMemcpyAsync(S.d_beta, b.data(), sizeof(double) * nh, cudaMemcpyHostToDevice, c->stream);
         if (e == cudaSuccess && !cf.empty())
-            e = cudaMemcpy(S.d_coef, cf.data(), sizeof(double) * cf.size(), cudaMemcpyHostToDevice);
-        if (e == cudaSuccess) e = cudaMemcpy(S.d_counter, counters, sizeof(int32_t) * 2, cudaMemcpyHostToDevice);
+            e = cudaMemcpyAsync(S.d_coef, cf.data(), sizeof(double) * cf.size(), cudaMemcpyHostToDevice, c->stream);
+        if (e == cudaSuccess) e = cudaMemcpyAsync(S.d_counter, counters, sizeof(int32_t) * 2, cudaMemcpyHostToDevice, c->stream);
     }
     const uint64_t vb = sizeof(double2) * uint64_t(dim) * R;
     for (int r : {S.b0, S.b1, S.b2})

@@ -869,3 +869,33 @@ def test_checkpoint_leaves_the_plain_products_scale_alone(junk, tmp_path):
         out.append((w, pr, c.cg(-5.0, v, inv_max=2, cg_max=20)[0]))
     for x, y in zip(*out):
         assert np.array_equal(x, y)
+
+
+@pytest.mark.parametrize("R,field", [(1, False), (16, True)])
+def test_contexts_made_behind_a_busy_legacy_stream(R, field):
+    """The first products of contexts created while the legacy default stream has work
+    queued: the counters, scales and table sources that creation uploads have landed
+    (the contexts' stream does not wait for the legacy one)."""
+    n = 14 if R == 16 else 12
+    gm, om = _chain_model(n, field)
+    rng = np.random.default_rng(7)
+    v = rng.standard_normal((gm.dim, R)) + 1j * rng.standard_normal((gm.dim, R))
+    ref = np.zeros_like(v)
+    for r in range(R):
+        col = np.zeros(gm.dim, dtype=np.complex128)
+        om.p_mltply_v3(np.ascontiguousarray(v[:, r]), col)
+        ref[:, r] = col
+    dv = torch.from_numpy(np.ascontiguousarray(v).reshape(-1)).cuda()
+    out = torch.zeros_like(dv)
+    busy = torch.zeros(1 << 26, device="cuda")
+    torch.cuda.synchronize()
+    for _ in range(20):
+        fresh, _ = _chain_model(n, field)
+        out.zero_()
+        torch.cuda.synchronize()
+        for _ in range(20):
+            busy.add_(1.0)
+        ctx = P.Context(fresh, R=R)
+        ctx.p_mltply_v3(dv, out)
+        assert rel(out.cpu().numpy().reshape(gm.dim, R), ref) <= 1e-12
+        ctx.close()
