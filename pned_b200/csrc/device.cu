@@ -152,7 +152,7 @@ __global__ void __launch_bounds__(kThreads) hv_xor_kernel(const __grid_constant_
         hv_epilogue<K, VPT>(a, s, r0, v, acc, scr, pcr, gsr, red);
     }
     block_reduce_store<K, VPT>(red, G, VPT, R, a.partials);
-    hv_finish(a);
+    if (K == 1 && VPT == 1) hv_finish(a);
 }
 
 // Tiled single-vector (R = 1) H.v on the S = 1/2 full basis, one pass of a
@@ -344,7 +344,7 @@ __global__ void __launch_bounds__(kThreads, BPS)
     }
     // static order: the block's sums over its tiles (same reduction order)
     if (!ctr) tile_sums_store<K>(red, s_red, a.partials + size_t(blockIdx.x) * K);
-    if (prog.last) hv_finish(a, smem);
+    if (K == 1 && prog.last) hv_finish(a, smem);
 }
 
 // Tiled multi-vector H.V (R > 1 interleaved vectors, S = 1/2 full basis), one
@@ -545,7 +545,6 @@ __global__ void __launch_bounds__(kThreads, 2) hv_tile_rv_kernel(const __grid_co
         chunk = s_next;
     }
     if (!ctr) block_reduce_store<K, VPT, true>(red, G, VPT, R, a.partials);
-    if (prog.last) hv_finish(a, smem);
 }
 
 // Mixed-radix (q > 2) variant: partner = s + offset, coefficient indexed by
@@ -616,7 +615,7 @@ __global__ void __launch_bounds__(kThreads) hv_radix_kernel(const __grid_constan
         hv_epilogue<K, VPT>(a, s, r0, v, acc, scr, pcr, gsr, red);
     }
     block_reduce_store<K, VPT>(red, G, VPT, R, a.partials);
-    hv_finish(a);
+    if (K == 1 && VPT == 1) hv_finish(a);
 }
 
 // Sums partials[nb][KR] in a fixed order into out[KR] (one block).
@@ -672,7 +671,7 @@ __global__ void __launch_bounds__(kThreads) dot_kernel(const double2 *__restrict
 // Lanczos.f90:111-130): alpha, beta recorded, the next scales set.  Two launches fewer a
 // step; N = 18 (everything in L2) is launch-bound.
 __global__ void __launch_bounds__(kThreads) residual_kernel(const double2 *__restrict__ W, const double2 *__restrict__ C,
-                                                            double2 *Rn, const double *__restrict__ sc,
+                                                            double2 *Rn, const double *sc /* tail.sc */,
                                                             const double2 *__restrict__ alpha, int64_t dim, int R,
                                                             int vpt, double2 *partials, const Finish fin,
                                                             const LanczosTail tail)
@@ -960,8 +959,7 @@ static cudaError_t launch_rv_t(const pned_model *m, const pned_model::TileSet &t
     const bool dyn = tile_dynamic(m, a, nblocks);
     HvArgs b = a;
     if (!dyn) b.tile_counter = nullptr;
-    else if (!a.fin.out &&
-             (e = cudaMemsetAsync(a.tile_counter, 0, sizeof(uint32_t) * kTileMaxPasses, st)) != cudaSuccess)
+    else if ((e = cudaMemsetAsync(a.tile_counter, 0, sizeof(uint32_t) * kTileMaxPasses, st)) != cudaSuccess)
         return e;
     size_t off = 0;
     for (size_t p = 0; p < ts.progs.size(); ++p) {
@@ -1070,12 +1068,12 @@ cudaError_t launch_hv(const pned_model *m, const HvArgs &a, int nblocks, cudaStr
 
 // Rows up to which the last block of the H.v kernel finishes the sums: the finish kernel's
 // single-block range, whose order of additions it keeps bit for bit (longer lists go through
-// two levels).  One column only: several columns take a block as many passes, and the finish
-// kernel is then as fast (N = 20, R = 4, 16 columns: 459 us a step against 360 us).
+// two levels).  One column only: one block adds several columns one after another, which takes
+// longer than the finish kernel's launch (N = 20, R = 4, 16 columns: 459 us a step with the
+// sums in the kernel, 360 us with the finish kernel).
 constexpr int64_t kFinishInKernel = 2048;
 
-cudaError_t launch_hv_sums(const pned_model *m, const HvArgs &a, int nblocks, double2 *out, cudaStream_t st,
-                           const TpsTail *tail, bool *in_kernel)
+cudaError_t launch_hv_sums(const pned_model *m, const HvArgs &a, int nblocks, double2 *out, cudaStream_t st)
 {
     const int64_t rows = hv_partials(m, a, nblocks);
     const int kr = a.K * a.R;
@@ -1084,7 +1082,6 @@ cudaError_t launch_hv_sums(const pned_model *m, const HvArgs &a, int nblocks, do
     // the S = 1 kernel (its block size varies) and the sector's segment kernel (at its register
     // limit: 1 % slower with the sums in it, N = 28) leave them to the finish kernels
     const bool in = a.fin.done && kr == 1 && !staged && !find_q3(m, a.R) && !sector_segments_on(m) && rows <= kFinishInKernel;
-    if (in_kernel) *in_kernel = in;
     if (in) {
         b.fin.base = a.partials;
         b.fin.out = out;
@@ -1095,7 +1092,6 @@ cudaError_t launch_hv_sums(const pned_model *m, const HvArgs &a, int nblocks, do
             b.tile_counter = b.fin.ctr;
             b.fin.nctr = kTileCounters;
         }
-        if (tail) b.tail = *tail;
         return launch_hv(m, b, nblocks, st);
     }
     b.fin.out = nullptr;

@@ -197,10 +197,8 @@ void session_release(pned_ctx *c);
 
 cudaError_t launch_hv(const pned_model *m, const HvArgs &a, int nblocks, cudaStream_t st);
 // H.v and its sums into out[K * R]: in the kernel where a.fin.done is given and the rows
-// are few, else by the finish kernels.  `tail`: what follows the sums when they are finished
-// in the kernel (*in_kernel is set then).
-cudaError_t launch_hv_sums(const pned_model *m, const HvArgs &a, int nblocks, double2 *out, cudaStream_t st,
-                           const TpsTail *tail = nullptr, bool *in_kernel = nullptr);
+// are few, else by the finish kernels.
+cudaError_t launch_hv_sums(const pned_model *m, const HvArgs &a, int nblocks, double2 *out, cudaStream_t st);
 // Raises a kernel's dynamic shared memory limit to 200 KB (once per kernel and device).
 cudaError_t allow_dynamic_smem(const void *kern, int device);
 // Device chosen by pned_set_device on this host thread.
@@ -445,41 +443,11 @@ __device__ __forceinline__ bool finish_last(const Finish &f, double2 *s_fin)
     return true;
 }
 
-// TPS step: alpha1 = Re<v|(L-H)v>, beta = ||(L-H)v||, coefficients as eval_phys_val; the
-// next scales.  s: the sums [4][R]; so: the observables' sums.
-__device__ __forceinline__ void tps_tail(const TpsTail &t, const double2 *s, int nobs, const double2 *so)
-{
-    const int k = *t.counter, R = t.R;
-    __syncthreads();
-    for (int r = int(threadIdx.x); r < R; r += int(blockDim.x)) {
-        const double a1 = s[0 * R + r].x;
-        const double be = sqrt(s[1 * R + r].x);
-        const double2 zero = make_double2(0.0, 0.0);
-        const double2 gw = t.first ? zero : s[2 * R + r], gv = t.first ? zero : s[3 * R + r];
-        t.alpha[(size_t)k * R + r] = t.L - a1;
-        t.beta[(size_t)k * R + r] = be;
-        double *cf = t.coef + ((size_t)k * R + r) * t.ncoef;
-        cf[0] = double(2 * (k + 1)) / a1;
-        cf[1] = t.L;
-        cf[2] = be;
-        cf[3] = t.L - a1;
-        cf[4] = t.L * gv.x - gw.x;   // Re(L <vg|v1> - <vg|v0>)
-        for (int o = 0; o < nobs; ++o) {
-            cf[5 + 2 * o] = so[(2 * o) * R + r].x;
-            cf[6 + 2 * o] = so[(2 * o + 1) * R + r].x;
-        }
-        t.gscp[r] = t.gsc[r];
-        t.gsc[r] = t.sc[r];
-        t.sc[r] = 1.0 / be;
-    }
-    __syncthreads();
-    if (threadIdx.x == 0) *t.counter = k + 1;
-}
-
-// End of an H.v kernel: every thread of every block, after its partial sums.
+// End of an H.v kernel for one vector and one sum (K * R = 1; instances for more leave it
+// out): every thread of every block, after its partial sums.
 __device__ __forceinline__ void hv_finish(const HvArgs &a, double2 *s_fin)
 {
-    if (finish_last(a.fin, s_fin) && a.tail.on) tps_tail(a.tail, a.fin.out, 0, nullptr);
+    finish_last(a.fin, s_fin);
 }
 __device__ __forceinline__ void hv_finish(const HvArgs &a)
 {

@@ -196,7 +196,7 @@ __global__ void __launch_bounds__(kThreads, 2) hv_qtile_kernel(const __grid_cons
         for (int w = 0; w < nw; ++w) sum = cadd(sum, sm[(size_t(w) * K + k) * R + r]);
         a.partials[((size_t)blockIdx.x * K + k) * R + r] = sum;
     }
-    if (prog.last) hv_finish(a, smem);
+    if (K == 1 && VPT == 1 && prog.last) hv_finish(a, smem);
 }
 
 // Tile set of the mixed-radix tiled kernel for R (null: the flat kernel runs).

@@ -861,7 +861,7 @@ __global__ void __launch_bounds__(kThreads, 2)
         mbar_wait(bar_v, phase ^ 1u);
         mbar_wait(bar_e, phase ^ 1u);
     }
-    if (prog.last) hv_finish(a, s_v);   // (own buffers as scratch: more static shared memory would take L1)
+    if (K == 1 && prog.last) hv_finish(a, s_v);   // (own buffers as scratch: more static shared memory would take L1)
 }
 
 void *tile_tma_encoder()

@@ -296,7 +296,7 @@ __global__ void __launch_bounds__(kThreads, 2)
     }
     if (!ctr) red[0] = cscale(sc * hs, red[0]);
     if (!ctr) x_sums_store<K>(red, s_red, lr, R, ch, a.partials + size_t(blk) * K * R);
-    if (prog.last) hv_finish(a, smem);   // the tile buffer is free behind the first barrier in there
+    if (K == 1 && prog.last) hv_finish(a, smem);   // the tile buffer is free behind the first barrier in there
 }
 
 const pned_model::XTileSet *find_xtiles(const pned_model *m, int R)

@@ -129,15 +129,6 @@ struct Finish {
     int rows, kr, nctr;
 };
 
-// Step epilogue of a TPS session, run behind the sums (see tps_tail).
-struct TpsTail {
-    int on, R, ncoef;
-    double L;
-    double *sc, *gsc, *gscp, *alpha, *beta, *coef;
-    int *counter;
-    int first;
-};
-
 // Per-call scalars: W = pc_r * P + sc_r * (H - shift) (sc_r * C); all from device memory.
 struct HvArgs {
     const double2 *C;       // input vectors (scaled by sc)
@@ -168,9 +159,8 @@ struct HvArgs {
     // written per tile ([tile][K]) instead of per block.  Null: the static
     // order (tile = block + k * grid) with per-block sums.
     uint32_t *tile_counter;
-    // sums finished in the kernel (last pass), and what follows them
+    // sums finished in the kernel (last pass; K * R = 1 only, see launch_hv_sums)
     Finish fin;
-    TpsTail tail;
     int64_t partials_cap;   // double2 slots available at `partials` (per-tile sums need sum(tiles) * K)
     int rv_chunk;           // multi-vector kernel, dynamic order: tiles per chunk (set by the launcher)
     // Sz sector (set by launch_hv from the model): index -> state, and the Lin

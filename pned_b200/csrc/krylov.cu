@@ -19,10 +19,43 @@ namespace pned {
 // step epilogues (one block, one thread per vector)
 // ---------------------------------------------------------------------------
 
-// TPS step whose sums the finish kernels made, and observables.
-__global__ void tps_epilogue(const TpsTail t, const double2 *__restrict__ s, int nobs, const double2 *__restrict__ so)
+// TPS: alpha1 = Re<v|(L-H)v>, beta = ||(L-H)v||, coefficients as eval_phys_val; the next
+// scales.  s: the sums [4][R]; so: the observables' sums.
+struct TpsStep {
+    int R, ncoef, nobs, first;
+    double L;
+    double *sc, *gsc, *gscp, *alpha, *beta, *coef;
+    int *counter;
+};
+__global__ void tps_epilogue(const TpsStep t, const double2 *__restrict__ s, const double2 *__restrict__ so)
 {
-    tps_tail(t, s, nobs, so);
+    __shared__ int k;
+    if (threadIdx.x == 0) k = *t.counter;
+    __syncthreads();
+    const int R = t.R, r = threadIdx.x;
+    if (r < R) {
+        const double a1 = s[0 * R + r].x;
+        const double be = sqrt(s[1 * R + r].x);
+        const double2 zero = make_double2(0.0, 0.0);
+        const double2 gw = t.first ? zero : s[2 * R + r], gv = t.first ? zero : s[3 * R + r];
+        t.alpha[(size_t)k * R + r] = t.L - a1;
+        t.beta[(size_t)k * R + r] = be;
+        double *cf = t.coef + ((size_t)k * R + r) * t.ncoef;
+        cf[0] = double(2 * (k + 1)) / a1;
+        cf[1] = t.L;
+        cf[2] = be;
+        cf[3] = t.L - a1;
+        cf[4] = t.L * gv.x - gw.x;   // Re(L <vg|v1> - <vg|v0>)
+        for (int o = 0; o < t.nobs; ++o) {
+            cf[5 + 2 * o] = so[(2 * o) * R + r].x;
+            cf[6 + 2 * o] = so[(2 * o + 1) * R + r].x;
+        }
+        t.gscp[r] = t.gsc[r];
+        t.gsc[r] = t.sc[r];
+        t.sc[r] = 1.0 / be;
+    }
+    __syncthreads();
+    if (threadIdx.x == 0) *t.counter = k + 1;
 }
 
 // Diagonal observables: <v|O v> and <g|O v>, v = sc C, g = gsc G.
@@ -303,11 +336,7 @@ static cudaError_t tps_step(pned_ctx *c, Session &S, bool first)
     a.err = c->flag;
     ctx_tile_args(c, a);
     if (S.ev_hv0) cudaEventRecord(S.ev_hv0, c->stream);
-    const TpsTail tail{1, R, S.ncoef, S.L, slot(c, kSlotSc), slot(c, kSlotGsc), slot(c, kSlotGscPrev), S.d_alpha,
-                       S.d_beta, S.d_coef, S.d_counter, first ? 1 : 0};
-    bool closed = false;   // the H.v kernel closes the step (no observables)
-    cudaError_t e = launch_hv_sums(c->m, a, c->nblocks, c->sums, c->stream, S.nobs ? nullptr : &tail, &closed);
-    closed = closed && !S.nobs;
+    cudaError_t e = launch_hv_sums(c->m, a, c->nblocks, c->sums, c->stream);
     if (S.ev_hv1) cudaEventRecord(S.ev_hv1, c->stream);
     for (int o = 0; o < S.nobs && e == cudaSuccess; ++o) {
         const DevObs &ob = S.obs[o];
@@ -318,8 +347,10 @@ static cudaError_t tps_step(pned_ctx *c, Session &S, bool first)
         e = cudaGetLastError();
         if (e == cudaSuccess) e = launch_finish(c->partials, c->nblocks, 2 * R, S.d_osum + 2 * o * R, c->stream);
     }
-    if (e == cudaSuccess && !closed) {
-        tps_epilogue<<<1, 32 * ((R + 31) / 32), 0, c->stream>>>(tail, c->sums, S.nobs, S.d_osum);
+    if (e == cudaSuccess) {
+        const TpsStep t{R, S.ncoef, S.nobs, first ? 1 : 0, S.L, slot(c, kSlotSc), slot(c, kSlotGsc),
+                        slot(c, kSlotGscPrev), S.d_alpha, S.d_beta, S.d_coef, S.d_counter};
+        tps_epilogue<<<1, 32 * ((R + 31) / 32), 0, c->stream>>>(t, c->sums, S.d_osum);
         e = cudaGetLastError();
     }
     const int og = S.b2;

@@ -361,7 +361,7 @@ struct pned_slots {
     double2 *partials = nullptr, *sums = nullptr, *scratch = nullptr;   // scratch: [R][n] phases + [R][nbond*4] dtab
     int64_t partials_cap = 0;        // double2 slots at `partials`
     uint32_t *tile_ctr = nullptr;    // tile counters of the dynamic tile order
-    uint32_t *fin_ctr = nullptr;     // block count and tile counters of kernels that finish their sums
+    uint32_t *fin_ctr = nullptr;     // block count of the residual kernel, which finishes its sums
     cudaGraphExec_t graph = nullptr;
     int64_t enqueued = 0;
     // R = 1: the batch's table and diagonal have the layout of a model's, so the
@@ -407,8 +407,6 @@ cudaError_t slot_step(pned_slots *S)
         a.slot_tables = R > 1;
         a.tile_counter = S->tile_ctr;
         a.partials_cap = S->partials_cap;
-        a.fin.done = S->fin_ctr;
-        a.fin.ctr = S->fin_ctr + 1;
         e = launch_hv_sums(&S->tm, a, S->nblocks, s4, S->stream);
     } else {
         SlotHvArgs a{};
@@ -624,8 +622,8 @@ extern "C" int pned_slots_create(const pned_model_desc *structure, int R, int ma
     S->partials_cap = std::max<int64_t>(S->partials_cap, (S->dim * R / 2048 + 1) * 2 * kMaxK * R / std::min(R, kXMaxVec));
     if (e == cudaSuccess) e = salloc(S.get(), &S->partials, size_t(S->partials_cap));
     if (e == cudaSuccess) e = cudaMalloc(&S->tile_ctr, sizeof(uint32_t) * kTileCounters);
-    if (e == cudaSuccess) e = cudaMalloc(&S->fin_ctr, sizeof(uint32_t) * (1 + kTileCounters));
-    if (e == cudaSuccess) e = cudaMemset(S->fin_ctr, 0, sizeof(uint32_t) * (1 + kTileCounters));
+    if (e == cudaSuccess) e = cudaMalloc(&S->fin_ctr, sizeof(uint32_t));
+    if (e == cudaSuccess) e = cudaMemset(S->fin_ctr, 0, sizeof(uint32_t));
     if (e == cudaSuccess) e = salloc(S.get(), &S->sums, size_t(12) * kMaxR);
     if (e == cudaSuccess) e = salloc(S.get(), &S->scratch, size_t(R) * 64 + size_t(R) * S->nbond * 4);
     if (e == cudaSuccess) e = cudaMemcpy(S->s1, hp.dsite1.data(), sizeof(int) * S->nbond, cudaMemcpyHostToDevice);
