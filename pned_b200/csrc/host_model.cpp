@@ -1015,6 +1015,10 @@ int plan_xtiles_for(const HostProgram &P, int R, int &lr, std::vector<XTilePass>
     // below 2^18 elements there are fewer tiles than resident blocks and a call is launch-bound:
     // the other kernels are as fast (N = 14, R = 16: 0.116 ms both)
     if (P.q != 2 || P.sector || P.n < 12 || R == 3 || double(P.dim) * R < double(1 << 18)) return PNED_ENOTSUP;
+    // R = 6: groups of two vectors, 32-byte runs, pay from 2^19 elements on (mTPQ step with a field:
+    // N = 16 53.6 against 49.3 us with the multi-vector kernel, N = 17 77.1 against 76.6, N = 18
+    // 121 against 137; without a field N = 17 62.2 against 69.8)
+    if (R == 6 && double(P.dim) * R < double(1 << 19)) return PNED_ENOTSUP;
     // Tiles of 2048 elements: up to 8 vectors of 2^(11 - lr) states.  A warp's global read
     // moves 128 bytes a wavefront only from whole lines, so groups are as wide as R divides
     // (8 vectors: 128-byte runs; N = 24, R = 16: 14.8 ms against 16.6 ms with groups of 4 and

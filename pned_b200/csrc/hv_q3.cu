@@ -274,12 +274,15 @@ cudaError_t launch_q3(const pned_model *m, const pned_model::Q3Set &qs, const Hv
 // The S = 1 passes for one vector (several: the kernel for any base runs, whose threads
 // share a term's decode over their vectors; N = 16, R = 4: 20.6 against 21.6 ms a step,
 // N = 12, R = 8: 0.41 against 0.52 ms): the largest tile whose two buffers, tables and index
-// arrays leave room for two blocks per SM.  False (any other base, an element that moves a
+// arrays leave room for two blocks per SM.  From 9 sites on: at 8 there are 81 tiles for 148
+// SMs, and the few items of a tile make its nine states a thread a serial chain (Lanczos step
+// 31.1 against 27.2 us, mTPQ step 35.9 against 25.4 us; N = 9: 36.2 against 52.8 and 42.4
+// against 52.7).  False (any other base, an element that moves a
 // digit by two, no room): the kernel for any base runs.
 bool ensure_q3(pned_model *m, int R)
 {
     const HostProgram &hp = m->hp;
-    if (hp.q != 3 || hp.sector || hp.n < 8 || hp.n > 20 || R != 1) return false;
+    if (hp.q != 3 || hp.sector || hp.n < 9 || hp.n > 20 || R != 1) return false;
     std::lock_guard<std::mutex> lock(m->rtiles_mu);
     if (m->q3.count(R)) return !m->q3[R].progs.empty();
     pned_model::Q3Set &qs = m->q3[R];

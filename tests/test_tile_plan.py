@@ -381,6 +381,22 @@ def test_class_tiled_plan_matches_every_flip_term(n, R, field):
     assert len(got) == len(r["xterms"]) and set(got) == want
 
 
+@pytest.mark.parametrize("n,R,runs", [(12, 16, False), (14, 16, True), (16, 2, False), (16, 3, False), (16, 4, True),
+                                      (16, 6, False), (18, 6, True), (18, 3, False)])
+def test_class_tiled_plan_runs_where_it_is_the_faster(n, R, runs):
+    """The class-tiled passes start at 2^18 elements, at 2^19 for six vectors (groups of two,
+    32-byte runs), and never for three."""
+    from pned_b200.lattice import cluster_for_sites
+    cl = cluster_for_sites(n)
+    X, skip, pt = P.build_xlocal(2, 0, CP.kitaev_heisenberg(0.6, 1.6))
+    d = P.ModelInput(n, 2, 0, cl.ipair, cl.ibond_type, X, skip, pt)
+    if runs:
+        assert api.xtile_plan_export(d, R)["passes"]
+    else:
+        with pytest.raises(P.PnedError):
+            api.xtile_plan_export(d, R)
+
+
 @pytest.mark.parametrize("L1,L2,k,low,field", [(3, 2, 5, 0, False), (3, 2, 6, 1, True), (2, 2, 4, 0, True), (3, 2, 7, 1, False)])
 def test_s1_members_match_every_radix_term(L1, L2, k, low, field):
     """The S = 1 kernel's members, followed through the thread's nine J states, the row
