@@ -141,9 +141,13 @@ int pned_model_plan(const pned_model *m, int R, int *tile_passes, int *partner_t
  * per thread 2^j_bits (fewer: fewer registers, more resident blocks; 4: tiles
  * of 4096 states, more flips inside the tile).  Re-plans at
  * once; call it between launches, not while other threads launch on the
- * model.  Used by the autotuner (pned_b200.tune).  plan NULL (and a model
- * whose plan was never set) takes the size's default: for R = 1 from 26
- * sites on, row_fixed_bits 5, window_bits 7, two passes, objective 1, stage
+ * model.  Sessions begun earlier keep their captured steps.  Used by the
+ * autotuner (pned_b200.tune).  plan NULL, a plan whose fields are all -1
+ * (stage 0; l1_carveout is taken as given), and a model whose plan was never
+ * set take the size's default: for several vectors the class-tiled kernel
+ * (not for 3, and from 2^18 elements on, 2^19 for 6; below, every field at its own
+ * default); for R = 1 from 26 sites on, with complex couplings the class-tiled kernel,
+ * with real ones row_fixed_bits 5, window_bits 7, two passes, objective 1, stage
  * 3, two terms in flight (the plan the autotuner picks on B200 at 26-30
  * sites); otherwise every field at its own default as described here.
  */
@@ -175,8 +179,8 @@ int pned_model_set_plan(pned_model *m, int R, const pned_tile_plan *plan);
  * (S = 1/2 full basis) that the planner builds for this model with row_bits row
  * bits a tile (8: the single-vector kernel, as pned_model_set_plan; fewer: the
  * multi-vector kernel's 256 / G rows), computed on the host without device
- * work; the default fixed row bits are min(row_bits, 8), and plan NULL with
- * row_bits 8 gives the model's default plan (from 26 sites on fixed 5, window
+ * work; the default fixed row bits are min(row_bits, 8), and plan NULL (or all
+ * fields -1) with row_bits 8 gives the model's default tile plan (from 26 sites on fixed 5, window
  * 7, 2 passes, objective 1).  out[0..cap)
  * receives int64 values, *len the full count: the number of flip terms X, X
  * records (xmask, pos4, tab, nb), the number of passes, and per pass (tbits, jb,

@@ -1238,8 +1238,8 @@ void build_tile_programs(pned_model *m)
     m->tprogs.clear();
     const HostProgram &hp = m->hp;
     std::vector<HostProgram::TilePass> passes;
-    // Without a plan set (pned_model_set_plan with NULL, or never called): from 26
-    // sites on, the plan the autotuner picks on B200 at 26-30 sites (tile bits that
+    // Without a plan set (pned_model_set_plan with NULL or a plan of defaults, or never
+    // called): from 26 sites on, the plan the autotuner picks on B200 at 26-30 sites (tile bits that
     // hold the most flip terms, 7 window bits, two passes, own rows by tensor copies,
     // two out-of-tile terms in flight); below, and for the fields a set plan leaves
     // at -1, the fewest partner tiles with a 10-bit window through the gather kernel.
@@ -1418,6 +1418,7 @@ extern "C" int pned_model_create(const pned_model_desc *desc, pned_model **out)
         if (e != cudaSuccess) return cuda_fail(e, "pned_model_create: sector segments");
     } else {
         build_tile_programs(m.get());
+        ensure_xtiles(m.get(), 1, false);   // one vector's default is settled here, as its plan's queries say
     }
     // coefficient table
     std::vector<double2> tab(std::max<size_t>(1, hp.table.size()));
@@ -1529,14 +1530,6 @@ extern "C" int pned_model_plan(const pned_model *m, int R, int *tile_passes, int
     return PNED_OK;
 }
 
-namespace pned {
-bool plan_default(const pned_tile_plan *p)
-{
-    return !p || (p->row_fixed_bits < 0 && p->window_bits < 0 && p->max_passes < 0 && p->j_bits < 0 &&
-                  p->stage_partner_tiles <= 0 && p->blocks_per_sm < 0 && p->objective < 0 && p->terms_in_flight < 0);
-}
-}  // namespace pned
-
 extern "C" int pned_model_set_plan(pned_model *m, int R, const pned_tile_plan *plan)
 {
     if (!m || pick_vpt(R) == 0) return fail(PNED_EINVAL, "pned_model_set_plan: bad arguments");
@@ -1546,10 +1539,10 @@ extern "C" int pned_model_set_plan(pned_model *m, int R, const pned_tile_plan *p
     cudaSetDevice(m->device);
     if (R == 1) {
         m->plan1 = plan ? *plan : pned_tile_plan{-1, -1, -1, -1, -1, -1, -1, -1, -1};
-        m->plan1_set = plan != nullptr;
+        m->plan1_set = !plan_default(plan);
         m->carveout = m->plan1.l1_carveout != 0;
         build_tile_programs(m);
-        switch_xtiles(m, 1, !plan);
+        switch_xtiles(m, 1, plan_default(plan));
         ensure_xtiles(m, 1, false);
         return PNED_OK;
     }

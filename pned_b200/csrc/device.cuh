@@ -20,6 +20,7 @@ struct DevBuf {
     ~DevBuf() { cudaFree(p); }
     bool upload(const void *src, size_t bytes)
     {
+        cudaFree(p);
         if (cudaMalloc(&p, bytes ? bytes : 1) != cudaSuccess) { p = nullptr; cudaGetLastError(); return false; }
         // waited for: kernels on streams that do not wait for the legacy one read it next
         return cudaMemcpyAsync(p, src, bytes, cudaMemcpyHostToDevice, cudaStreamPerThread) == cudaSuccess &&
@@ -217,8 +218,6 @@ size_t rtile_smem(const pned_model *m, int R, bool slot_tables);
 bool ensure_xtiles(pned_model *m, int R, bool slot_tables);
 const pned_model::XTileSet *find_xtiles(const pned_model *m, int R);
 void switch_xtiles(pned_model *m, int R, bool on);
-// No plan, or one whose every field asks for the default.
-bool plan_default(const pned_tile_plan *p);
 int64_t xtile_rows(const pned_model *m, const pned_model::XTileSet &xs, int R, int nblocks, bool dynamic);
 cudaError_t launch_xtile(const pned_model *m, const pned_model::XTileSet &xs, const HvArgs &a, int nblocks,
                          cudaStream_t st);

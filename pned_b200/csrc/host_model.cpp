@@ -726,6 +726,12 @@ int plan_tiles(const HostProgram &P, int tbits, int jb, int fixed, int window_bi
     return PNED_OK;
 }
 
+bool plan_default(const pned_tile_plan *p)
+{
+    return !p || (p->row_fixed_bits < 0 && p->window_bits < 0 && p->max_passes < 0 && p->j_bits < 0 &&
+                  p->stage_partner_tiles <= 0 && p->blocks_per_sm < 0 && p->objective < 0 && p->terms_in_flight < 0);
+}
+
 // ---------------------------------------------------------------------------
 // Planner of the class-tiled kernel
 // ---------------------------------------------------------------------------
@@ -1251,10 +1257,10 @@ extern "C" int pned_tile_plan_export(const pned_model_desc *d, int row_bits, con
     if (pl.max_passes > kTileMaxPasses || pl.window_bits > 30 || pl.row_fixed_bits > 8 || pl.j_bits > kTileMaxJB ||
         pl.j_bits == 0 || pl.objective > 1)
         return fail(PNED_EINVAL, "pned_tile_plan_export: plan out of range");
-    // the defaults of the model's own single-vector plan: with no plan, from
-    // kTileBigSites sites on, the tuned tensor-copy plan (5 fixed row bits,
+    // the defaults of the model's own single-vector plan: with no plan or a plan of
+    // defaults, from kTileBigSites sites on, the tuned tensor-copy plan (5 fixed row bits,
     // window 7, 2 passes, most terms inside the tile)
-    const bool big = !plan && row_bits == 8 && P.n >= kTileBigSites;
+    const bool big = plan_default(plan) && row_bits == 8 && P.n >= kTileBigSites;
     const int fixed = big ? 5 : std::min(row_bits, pl.row_fixed_bits >= 0 ? pl.row_fixed_bits : 8);
     const int window = big ? 7 : (pl.window_bits >= 0 ? pl.window_bits : kTileWindowBits);
     const int mp = big ? 2 : (pl.max_passes > 0 ? pl.max_passes : kTileMaxPasses);

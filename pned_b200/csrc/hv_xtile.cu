@@ -359,7 +359,12 @@ bool ensure_xtiles(pned_model *m, int R, bool slot_tables)
         xs.groups += t.groups;
         xs.progs.push_back(std::move(T));
     }
-    if (!xs.mem.upload(tsrc.data(), sizeof(uint16_t) * tsrc.size())) { xs.progs.clear(); return false; }
+    if (!xs.mem.upload(tsrc.data(), sizeof(uint16_t) * tsrc.size())) {   // no room now: the next context asks again
+        xs.progs.clear();
+        xs.groups = 0;
+        xs.built = false;
+        return false;
+    }
     const uint16_t *src = static_cast<const uint16_t *>(xs.mem.p);
     for (auto &T : xs.progs) {
         T->tsrc = src;

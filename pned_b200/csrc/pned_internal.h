@@ -189,6 +189,8 @@ int plan_qtiles(const HostProgram &P, int k, int low, std::vector<QTilePass> &pa
 // The same passes (q == 3) as hv_q3.cu takes them; PNED_ENOTSUP for elements that move a
 // digit by two.
 int plan_q3(const HostProgram &P, int k, int low, std::vector<Q3Pass> &passes);
+// No plan, or one whose every field asks for the default (l1_carveout apart).
+bool plan_default(const pned_tile_plan *p);
 int plan_tiles(const HostProgram &P, int tbits, int jb, int fixed, int window_bits, int max_passes,
                std::vector<HostProgram::TilePass> &out, int objective = 0);
 

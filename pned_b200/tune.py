@@ -8,8 +8,8 @@ kernel also takes the rows per thread (2^j_bits: 2048-state tiles at 3,
 4096-state tiles at 4) and the resident blocks per SM.  Which combination is fastest
 depends on the lattice, the vector count and the device, so the tuner times
 the H.V of the actual model over a small candidate set and keeps the
-fastest.  Results are cached in-process per (lattice, terms, R, device), and
-optionally in a JSON file.
+fastest.  Results are cached in-process per (candidate set, lattice, terms, real or
+complex couplings, R, device), and optionally in a JSON file.
 """
 from __future__ import annotations
 
@@ -50,6 +50,8 @@ CANDIDATES_R = [(-1, -1, -1), (0, 6, 2), (0, 8, 2), (0, 10, 2), (1, 10, 2), (3, 
 # the library's own default: from 26 sites on, complex couplings run the class-tiled kernel
 DEFAULT = (-1, -1, -1, -1)
 DEFAULT_DIM = 1 << 26
+# counts the sets of kernels and candidates that a cached plan was the fastest of
+VERSION = 2
 
 _cache: dict = {}
 
@@ -65,7 +67,8 @@ def _device_name():
 
 def _key(model, R):
     d = model.desc
-    return f"n{d.n}-q{d.q}-b{d.n_bonds}-t{model.n_terms}-ip{hash(d._ipair.tobytes()) & 0xffffffff:08x}-R{R}"
+    # real and complex couplings run different kernels under one plan
+    return f"v{VERSION}-n{d.n}-q{d.q}-b{d.n_bonds}-t{model.n_terms}-{'r' if model.real else 'c'}-ip{hash(d._ipair.tobytes()) & 0xffffffff:08x}-R{R}"
 
 
 def _time_hv(ctx, v1, v0, reps):

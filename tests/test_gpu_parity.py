@@ -899,3 +899,23 @@ def test_contexts_made_behind_a_busy_legacy_stream(R, field):
         ctx.p_mltply_v3(dv, out)
         assert rel(out.cpu().numpy().reshape(gm.dim, R), ref) <= 1e-12
         ctx.close()
+
+
+@pytest.mark.parametrize("field", [False, True])
+def test_single_vector_default_plan_is_one_plan(field):
+    """26 sites: the plan of a fresh model, with a context, after a plan of its own and a plan
+    of defaults is the same (real couplings: tensor copies; complex ones: class-tiled)."""
+    from pned_b200 import _capi
+    from pned_b200.lattice import cluster_for_sites
+    import ctypes as C
+    gm = P.Model.from_couplings(cluster_for_sites(26), KHGH if field else KH, field=FIELD if field else None)
+    first = gm.plan(1)
+    assert first["staging"] == (0 if field else 3) and first["tile_passes"] == 2
+    ctx = P.Context(gm, R=1)
+    assert gm.plan(1) == first
+    assert gm.set_plan(1, 5, 10, 2, 3) != first
+    defaults = _capi.TilePlan(-1, -1, -1, -1, 1, 0, -1, -1, -1)
+    P.api.check(P.api.lib().pned_model_set_plan(gm._h, 1, C.byref(defaults)))
+    assert gm.plan(1) == first
+    ctx.close()
+    gm.close()

@@ -319,6 +319,41 @@ def test_default_plan_below_26_sites_is_the_gather_plan():
     assert api.tile_plan_export(d) == api.tile_plan_export(d, 8, 10, -1, 3, objective=0)
 
 
+@pytest.mark.parametrize("n", [18, 26, 28])
+def test_a_plan_of_defaults_is_no_plan(n):
+    """A plan whose every field is -1 gives the plan that no plan gives, on both sides of
+    the 26-site line (the single-vector plan is the gather kernel's below it and the
+    tensor-copy kernel's from it on); one set field makes it a plan of its own."""
+    import ctypes as C
+    from pned_b200 import _capi
+    from pned_b200.lattice import cluster_for_sites
+    cl = cluster_for_sites(n)
+    X, skip, pt = P.build_xlocal(2, 0, CP.kitaev_heisenberg(0.6, 1.6))
+    d = P.ModelInput(n, 2, 0, cl.ipair, cl.ibond_type, X, skip, pt)
+
+    def export(plan):
+        buf, m = np.zeros(100000, dtype=np.int64), C.c_int64(0)
+        P.api.check(P.api.lib().pned_tile_plan_export(C.byref(d.c), 8, None if plan is None else C.byref(plan),
+                                                      buf.ctypes.data_as(C.POINTER(C.c_int64)), buf.size, C.byref(m)))
+        assert m.value <= buf.size
+        return buf[:m.value].tolist()
+
+    none = export(None)
+    assert export(_capi.TilePlan(-1, -1, -1, -1, 1, 0, -1, -1, -1)) == none
+    assert export(_capi.TilePlan(-1, -1, -1, -1, 0, -1, -1, -1, -1)) == none
+    assert export(_capi.TilePlan(3, 6, 1, 2, 1, 0, -1, -1, -1)) != none
+
+
+def test_tuned_plans_are_kept_apart_by_coupling_type_and_candidate_set():
+    """The tuner's key tells real from complex couplings (their default kernels differ) and
+    names the candidate set, so a cache file written for another one is not used."""
+    from types import SimpleNamespace
+    from pned_b200 import tune
+    d = SimpleNamespace(n=26, q=2, n_bonds=39, _ipair=np.arange(78, dtype=np.int32))
+    keys = [tune._key(SimpleNamespace(desc=d, n_terms=39, real=r), 1) for r in (True, False)]
+    assert keys[0] != keys[1] and all(k.startswith(f"v{tune.VERSION}-") for k in keys)
+
+
 XTILE_CASES = [(14, 16, True), (16, 4, False), (18, 2, True), (26, 1, True), (18, 4, True), (18, 6, False), (20, 8, True),
                (28, 1, False), (24, 12, False), (24, 16, True)]
 
