@@ -1072,6 +1072,13 @@ cudaError_t launch_hv(const pned_model *m, const HvArgs &a, int nblocks, cudaStr
 // longer than the finish kernel's launch (N = 20, R = 4, 16 columns: 459 us a step with the
 // sums in the kernel, 360 us with the finish kernel).
 constexpr int64_t kFinishInKernel = 2048;
+// The flat kernels run a block for every 256 states, so from the second wave of blocks on
+// (four on an SM) each one's fence in front of its count delays the blocks behind it, which
+// costs more than the finish kernel's launch (Lanczos step, sector of N = 20, 722 blocks: 35.2 us
+// with the sums in the kernel, 33.8 us with the finish kernel; sector of 14 S = 1 sites, 1184
+// blocks: 118 against 114 us; N = 18, 190 blocks: 18.8 against 19.3 us).  The tiled kernels'
+// blocks stay for all their tiles.
+constexpr int kFlatBlocksPerSM = 4;
 
 cudaError_t launch_hv_sums(const pned_model *m, const HvArgs &a, int nblocks, double2 *out, cudaStream_t st)
 {
@@ -1081,7 +1088,9 @@ cudaError_t launch_hv_sums(const pned_model *m, const HvArgs &a, int nblocks, do
     HvArgs b = a;
     // the S = 1 kernel (its block size varies) and the sector's segment kernel (at its register
     // limit: 1 % slower with the sums in it, N = 28) leave them to the finish kernels
-    const bool in = a.fin.done && kr == 1 && !staged && !find_q3(m, a.R) && !sector_segments_on(m) && rows <= kFinishInKernel;
+    const bool flat = !find_xtiles(m, a.R) && !(a.R == 1 && !m->tprogs.empty() && m->use_tile) && !find_qtiles(m, a.R);
+    const bool in = a.fin.done && kr == 1 && !staged && !find_q3(m, a.R) && !sector_segments_on(m) &&
+                    rows <= (flat ? std::min<int64_t>(kFinishInKernel, kFlatBlocksPerSM * m->nsm) : kFinishInKernel);
     if (in) {
         b.fin.base = a.partials;
         b.fin.out = out;
