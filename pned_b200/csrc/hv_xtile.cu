@@ -326,6 +326,11 @@ bool ensure_xtiles(pned_model *m, int R, bool slot_tables)
     // the sign of the Ritz vector that vec12 finds turns on the last bit of alpha and beta, so
     // another order may return -x where a caller had x.
     if (R == 1 && (m->real_coef || hp.n < kTileBigSites)) return false;
+    // Slot tables are staged per vector of the group, so a call needs more tiles to pay: 2^19
+    // elements (step of 4 slots: N = 16 52.8 against 51.2 us with the multi-vector kernel, N = 18
+    // 98.5 against 114.6), and for 6 slots, groups of two, 2^22 (N = 18 189 against 159 us, N = 20
+    // 543 against 642).
+    if (slot_tables && double(hp.dim) * R < double(R == 6 ? 1 << 22 : 1 << 19)) return false;
     std::lock_guard<std::mutex> lock(m->rtiles_mu);
     pned_model::XTileSet &xs = m->xtiles[R];
     if (xs.off || xs.built) return !xs.off && !xs.progs.empty();

@@ -260,3 +260,13 @@ def test_serving_results_alone_and_in_the_mix():
                 for got in (r, p):
                     check_chain(np.asarray(got["salpha"][k]), np.asarray(got["sbeta"][k]), ref, others, e0, q.steps,
                                 min_prefix=10)
+
+
+@pytest.mark.parametrize("n,R,states", [(16, 6, 256), (18, 6, 256), (20, 6, 1024), (14, 12, 128), (16, 12, 512)])
+def test_slot_batches_take_the_class_tiled_kernel_where_it_is_the_faster(n, R, states):
+    """States a tile on both sides of the slot rule (2^19 elements, 2^22 for six slots): the
+    class-tiled kernel holds 2048 elements of 2 or 4 vectors, the multi-vector one 256 or 128
+    states."""
+    sb = P.SlotBatch(P.ModelInput.structure(cluster_for_sites(n)), R, 4)
+    assert sb.plan()["tile_states"] == states
+    sb.close()
