@@ -1101,7 +1101,10 @@ cudaError_t launch_hv_sums(const pned_model *m, const HvArgs &a, int nblocks, do
             b.tile_counter = b.fin.ctr;
             b.fin.nctr = kTileCounters;
         }
-        return launch_hv(m, b, nblocks, st);
+        const cudaError_t e = launch_hv(m, b, nblocks, st);
+        // a pass that could not be launched leaves its predecessors' counters standing
+        if (e != cudaSuccess) cudaMemsetAsync(a.fin.done, 0, sizeof(uint32_t) * (1 + kTileCounters), st);
+        return e;
     }
     b.fin.out = nullptr;
     cudaError_t e = launch_hv(m, b, nblocks, st);
