@@ -1,5 +1,5 @@
-// Tiled S = 1 H.V (base 3, full basis, R interleaved vectors): the kernel, its launcher
-// and the tile sets built per model and R.
+// Tiled S = 1 H.v (base 3, full basis, one vector): the kernel, its launcher and the tile
+// sets built per model.
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -37,7 +37,7 @@ __device__ __forceinline__ void q3_apply(const double2 *ct, const double2 (&w)[k
 }
 
 // One pass: a tile is the 3^k states of k sites; thread t owns the 9 states of the two J
-// sites (local digits 0 and 1) for one setting of the others and one vector.  Members with
+// sites (local digits 0 and 1) for one setting of the others.  Members with
 // the same offset outside J share their nine partner rows (a class, as in hv_xtile.cu), and
 // their J part is a fixed register shift, so a term costs one row read and two products a
 // state; the kernel for any base (hv_qtile.cu) reads a coefficient and decodes the pair
@@ -47,15 +47,15 @@ __device__ __forceinline__ void q3_apply(const double2 *ct, const double2 (&w)[k
 // passes that move 10 GB).  H.v of one vector: N = 18 50.2 -> 32 ms, N = 16 5.52 -> 3.68 ms,
 // N = 14 with a field 1.15 -> 0.64 ms, N = 12 0.120 -> 0.089 ms.  Rows and the epilogue's
 // P or W and diagonal come in by cp.async in global order; local slots are nine apart from
-// lane to lane, so the 16-byte reads have no bank conflicts (vectors `vs` slots apart).
+// lane to lane, so the 16-byte reads have no bank conflicts.
 template <bool RC, bool RD, int K>
 __global__ void __launch_bounds__(kQ3Threads, 2) hv_q3_kernel(const __grid_constant__ Q3Program prog, const HvArgs a)
 {
     extern __shared__ double2 smem[];
-    const int R = a.R, nt = prog.nt, vs = prog.vs, nth = int(blockDim.x), tid = int(threadIdx.x);
-    double2 *s_v = smem;                           // [R][vs]
-    double2 *s_pw = s_v + size_t(vs) * R;          // rows of P or W, laid out as s_v
-    double2 *s_tab = s_pw + size_t(vs) * R;
+    const int nt = prog.nt, nth = int(blockDim.x), tid = int(threadIdx.x);
+    double2 *s_v = smem;                           // [nt]
+    double2 *s_pw = s_v + nt;                      // rows of P or W, laid out as s_v
+    double2 *s_tab = s_pw + nt;
     double *s_d = reinterpret_cast<double *>(s_tab + prog.ntab);             // [nt] real diagonal (first pass)
     uint32_t *s_goff = reinterpret_cast<uint32_t *>(s_d + (RD ? nt : 0));    // [nt] global offset of local slot
     uint16_t *s_slot = reinterpret_cast<uint16_t *>(s_goff + nt);            // [nt] local slot in global order
@@ -75,10 +75,8 @@ __global__ void __launch_bounds__(kQ3Threads, 2) hv_q3_kernel(const __grid_const
     double2 red[K];
 #pragma unroll
     for (int k = 0; k < K; ++k) red[k] = make_double2(0.0, 0.0);
-    // an item: vector r of the states 9 t .. 9 t + 8; a thread's items all have the same vector
-    // (the block size is a multiple of R)
-    const int nitems = nt / kQ3States * R, r = tid % R;
-    const double sc = a.sc[r], pc = a.pc ? a.pc[r] : 0.0, gs = a.gsc ? a.gsc[r] : 0.0;
+    const int nitems = nt / kQ3States;   // item t: the states 9 t .. 9 t + 8
+    const double sc = a.sc[0], pc = a.pc ? a.pc[0] : 0.0, gs = a.gsc ? a.gsc[0] : 0.0;
     const double2 *pw_src = prog.first ? a.P : a.W;
     __shared__ uint32_t s_base;
     for (int64_t tile = blockIdx.x; tile < prog.ntiles; tile += gridDim.x) {
@@ -94,15 +92,15 @@ __global__ void __launch_bounds__(kQ3Threads, 2) hv_q3_kernel(const __grid_const
         }
         __syncthreads();
         const uint32_t base = s_base;
-        for (int i = tid; i < nt * R; i += nth) {
-            const int l = s_slot[i / R];
-            cp_async16(s_v + r * vs + l, a.C + size_t(base + s_goff[l]) * R + r);
+        for (int i = tid; i < nt; i += nth) {
+            const int l = s_slot[i];
+            cp_async16(s_v + l, a.C + (base + s_goff[l]));
         }
         cp_async_commit();
         if (pw_src)
-            for (int i = tid; i < nt * R; i += nth) {
-                const int l = s_slot[i / R];
-                cp_async16(s_pw + r * vs + l, pw_src + size_t(base + s_goff[l]) * R + r);
+            for (int i = tid; i < nt; i += nth) {
+                const int l = s_slot[i];
+                cp_async16(s_pw + l, pw_src + (base + s_goff[l]));
             }
         if (RD && prog.first)
             for (int i = tid; i < nt; i += nth) {
@@ -115,8 +113,7 @@ __global__ void __launch_bounds__(kQ3Threads, 2) hv_q3_kernel(const __grid_const
         bool landed = false;   // the epilogue's rows
         for (int it = tid; it < nitems || !landed; it += nth) {
             const bool on = it < nitems;
-            const int t9 = on ? it / R * kQ3States : 0;
-            const double2 *sv = s_v + r * vs;
+            const int t9 = on ? it * kQ3States : 0;
             uint32_t dig = 0;   // the other digits, 2 bits each (digit 2 + i at bits 2 i)
             {
                 int x = t9 / kQ3States;
@@ -133,7 +130,7 @@ __global__ void __launch_bounds__(kQ3Threads, 2) hv_q3_kernel(const __grid_const
                 const Q3Sub S = prog.s[m];
                 if (S.first) {
                     // an offset that leaves the tile belongs to zero coefficients: clamped
-                    const double2 *p = sv + min(max(t9 + S.loff, 0), nt - kQ3States);
+                    const double2 *p = s_v + min(max(t9 + S.loff, 0), nt - kQ3States);
 #pragma unroll
                     for (int j = 0; j < kQ3States; ++j) w[j] = p[j];
                 }
@@ -165,13 +162,12 @@ __global__ void __launch_bounds__(kQ3Threads, 2) hv_q3_kernel(const __grid_const
             double2 g[K >= 4 ? kQ3States : 1];
             if (K >= 4 && prog.last && a.G) {
 #pragma unroll
-                for (int j = 0; j < kQ3States; ++j) g[j] = __ldcs(a.G + size_t(base + s_goff[t9 + j]) * R + r);
+                for (int j = 0; j < kQ3States; ++j) g[j] = __ldcs(a.G + (base + s_goff[t9 + j]));
             }
 #pragma unroll
             for (int j = 0; j < kQ3States; ++j) {
                 const uint32_t st = base + s_goff[t9 + j];
-                const size_t e = size_t(st) * R + r;
-                const double2 v = sv[t9 + j];
+                const double2 v = s_v[t9 + j];
                 double2 hsum = acc[j];
                 if (prog.first) {
                     if (RD) {
@@ -187,12 +183,12 @@ __global__ void __launch_bounds__(kQ3Threads, 2) hv_q3_kernel(const __grid_const
                 const double2 hv = cscale(sc, hsum);
                 double2 out = hv;
                 if (pw_src) {
-                    const double2 p = s_pw[r * vs + t9 + j];
+                    const double2 p = s_pw[t9 + j];
                     const double f = prog.first ? pc : 1.0;
                     out.x = fma(f, p.x, out.x);
                     out.y = fma(f, p.y, out.y);
                 }
-                __stcs(a.W + e, out);
+                __stcs(a.W + st, out);
                 const double2 vv = cscale(sc, v);
                 red[0] = cadd(red[0], cconjmul(vv, hv));
                 if (!prog.last) continue;
@@ -211,16 +207,14 @@ __global__ void __launch_bounds__(kQ3Threads, 2) hv_q3_kernel(const __grid_const
 #pragma unroll
     for (int k = 0; k < K; ++k) sm[tid * K + k] = red[k];
     __syncthreads();
-    const int g = tid / R, n = nth / R;
     for (int w = kQ3Threads / 2; w > 0; w >>= 1) {
-        if (w < n && g < w && g + w < n) {
+        if (w < nth && tid < w && tid + w < nth) {
 #pragma unroll
-            for (int k = 0; k < K; ++k) sm[tid * K + k] = cadd(sm[tid * K + k], sm[(tid + w * R) * K + k]);
+            for (int k = 0; k < K; ++k) sm[tid * K + k] = cadd(sm[tid * K + k], sm[(tid + w) * K + k]);
         }
         __syncthreads();
     }
-    for (int idx = tid; idx < K * R; idx += nth)
-        a.partials[size_t(blockIdx.x) * K * R + idx] = sm[(idx % R) * K + idx / R];
+    if (tid < K) a.partials[size_t(blockIdx.x) * K + tid] = sm[tid];
 }
 
 const pned_model::Q3Set *find_q3(const pned_model *m, int R)
@@ -247,7 +241,7 @@ static cudaError_t launch_q3_t(const pned_model *m, const pned_model::Q3Set &qs,
     const int grid = q3_grid(m, qs, nblocks);
     HvArgs b = a;
     for (size_t p = 0; p < qs.progs.size(); ++p) {
-        b.partials = a.partials + size_t(p) * grid * K * a.R;
+        b.partials = a.partials + size_t(p) * grid * K;
         kern<<<grid, qs.threads, qs.smem, st>>>(*qs.progs[p], b);
         e = cudaGetLastError();
         if (e != cudaSuccess) return e;
@@ -274,11 +268,11 @@ cudaError_t launch_q3(const pned_model *m, const pned_model::Q3Set &qs, const Hv
 // The S = 1 passes for one vector (several: the kernel for any base runs, whose threads
 // share a term's decode over their vectors; N = 16, R = 4: 20.6 against 21.6 ms a step,
 // N = 12, R = 8: 0.41 against 0.52 ms): the largest tile whose two buffers, tables and index
-// arrays leave room for two blocks per SM.  From 9 sites on: at 8 there are 81 tiles for 148
-// SMs, and the few items of a tile make its nine states a thread a serial chain (Lanczos step
-// 31.1 against 27.2 us, mTPQ step 35.9 against 25.4 us; N = 9: 36.2 against 52.8 and 42.4
-// against 52.7).  False (any other base, an element that moves a
-// digit by two, no room): the kernel for any base runs.
+// arrays leave room for two blocks per SM.  From 9 sites on: at 8 a tile is 729 states, 81
+// items, so nine blocks of three warps run, each thread's nine states one after another
+// (Lanczos step 31.1 against 27.2 us with the kernel for any base, mTPQ step 35.9 against
+// 25.4 us; N = 9, 243 items: 36.2 against 52.8 and 42.4 against 52.7).  False (any other base,
+// an element that moves a digit by two, no room): the kernel for any base runs.
 bool ensure_q3(pned_model *m, int R)
 {
     const HostProgram &hp = m->hp;
@@ -289,23 +283,15 @@ bool ensure_q3(pned_model *m, int R)
     int64_t pw[32];
     pw[0] = 1;
     for (int i = 1; i <= hp.n; ++i) pw[i] = pw[i - 1] * 3;
-    // slots between vectors: the 8 lanes of a 16-byte read phase (vectors first, then items
-    // nine apart) fall on distinct banks
-    auto stride = [&](int nt) {
-        const int want = R == 2 ? 4 : (R == 4 ? 2 : 1);
-        int v = nt;
-        while (v % 8 != want) ++v;
-        return v;
-    };
     auto smem_of = [&](int k, int ntab) {
         const int nt = int(pw[k]);
-        return sizeof(double2) * (2 * size_t(stride(nt)) * R + ntab) + size_t(nt) * (sizeof(double) + 6) + 16;
+        return sizeof(double2) * (2 * size_t(nt) + ntab) + size_t(nt) * (sizeof(double) + 6) + 16;
     };
     int k = 3;
-        while (k + 1 <= std::min(hp.n - 2, 7) && smem_of(k + 1, kQ3MaxTab) <= 112 * 1024) ++k;
+    while (k + 1 <= std::min(hp.n - 2, 7) && smem_of(k + 1, kQ3MaxTab) <= 112 * 1024) ++k;
     if (smem_of(k, kQ3MaxTab) > 112 * 1024) return false;
     std::vector<Q3Pass> passes;
-    if (plan_q3(hp, k, R == 1 ? 1 : 0, passes) != PNED_OK || passes.size() > size_t(kQTileMaxPasses)) return false;
+    if (plan_q3(hp, k, 1, passes) != PNED_OK || passes.size() > size_t(kQTileMaxPasses)) return false;
     int ntab = 1;
     for (size_t p = 0; p < passes.size(); ++p) {
         const Q3Pass &ps = passes[p];
@@ -313,7 +299,6 @@ bool ensure_q3(pned_model *m, int R)
         std::unique_ptr<Q3Program> T(new Q3Program());
         T->k = k;
         T->nt = int(pw[k]);
-        T->vs = stride(T->nt);
         T->nouter = int(ps.outer.size());
         T->nsub = int(ps.subs.size());
         T->ntab = int(ps.tsrc.size());
@@ -336,13 +321,11 @@ bool ensure_q3(pned_model *m, int R)
         qs.progs.push_back(std::move(T));
     }
     qs.smem = smem_of(k, ntab);
-    // threads: the items in as few rounds of at most 256 as they need, a multiple of 32 and of R
-    const int items = int(pw[k]) / kQ3States * R, rounds = (items + kQ3Threads - 1) / kQ3Threads;
-    int lcm = 32;
-    while (lcm % R) lcm += 32;
-    qs.threads = std::min(kQ3Threads / lcm * lcm, ((items + rounds - 1) / rounds + lcm - 1) / lcm * lcm);
+    // threads: the items in as few rounds of at most 256 as they need, a multiple of 32
+    const int items = int(pw[k]) / kQ3States, rounds = (items + kQ3Threads - 1) / kQ3Threads;
+    qs.threads = ((items + rounds - 1) / rounds + 31) / 32 * 32;
     // the block sums use the tile buffers
-    if (size_t(qs.threads) * kMaxK > size_t(2) * stride(int(pw[k])) * R) { qs.progs.clear(); return false; }
+    if (size_t(qs.threads) * kMaxK > size_t(2) * size_t(pw[k])) { qs.progs.clear(); return false; }
     return true;
 }
 

@@ -167,7 +167,7 @@ __global__ void __launch_bounds__(kThreads, 2)
                 const int64_t st = int64_t(base | prog.jexp[j]);
                 cp_async8(s_d + tid + kThreads * j,
                           static_cast<const double *>(a.diag) + (SLOT ? st * R + rg : st));
-        }
+            }
         }
         cp_async_commit();
     };

@@ -80,7 +80,7 @@ struct TileProgram {
 
 // One pass of the S = 1 kernel (see Q3Sub).
 struct Q3Program {
-    int k, nt, vs, nouter, nsub, ntab, first, last;
+    int k, nt, nouter, nsub, ntab, first, last;
     int64_t ntiles;
     uint32_t spow[8], rank[8];      // 3^site of local digit i, and its weight among the tile's sites
     uint32_t opow[32];
