@@ -784,6 +784,9 @@ def test_class_tiled_and_in_kernel_sums_parity(n, R, field):
     calls in a row: the counters that a kernel leaves for the next are zero."""
     gm, om = _chain_model(n, field)
     ctx = P.Context(gm, R=R)
+    if R > 1:   # the class-tiled kernel, one pass
+        assert gm.plan(R)["tile_states"] == 2048 // {2: 2, 4: 4, 6: 2, 8: 8, 12: 4, 16: 8}[R]
+        assert gm.plan(R)["tile_passes"] == 1
     rng = np.random.default_rng(n * 17 + R)
     D = gm.dim
     v1 = (rng.standard_normal((D, R)) + 1j * rng.standard_normal((D, R))).astype(np.complex128)
@@ -919,3 +922,129 @@ def test_single_vector_default_plan_is_one_plan(field):
     assert gm.plan(1) == first
     ctx.close()
     gm.close()
+
+
+def _odd_model(n, form):
+    """Models of n sites that reach the class-tiled kernel's rarer forms: "complex" (Gamma and
+    a field), "complete" (nine sites all coupled: members without a variant) and "diagonal"
+    (local matrices with an imaginary diagonal); and the same shifted for mTPQ."""
+    from tests.test_tile_plan import _complete_graph
+    if form == "complete":
+        ipair, bt = _complete_graph(n, 9)
+    else:
+        ipair = np.array([[i + 1, i + 2] for i in range(n - 1)] + [[1, n // 2]], dtype=np.int32).reshape(-1)
+        bt = np.array([1 + i % 3 for i in range(n)], dtype=np.int32)
+    X, skip, pt = P.build_xlocal(2, 0, KHGH, field=FIELD)
+    X = X.copy()
+    if form == "diagonal":
+        for t in range(9):
+            for i in range(4):
+                X[t, i, i] += 0.01j * (i + 1) * (t + 1)
+    return (P.Model(n, 2, 0, ipair, bt, X, skip, pt), O.Model(n, 2, 0, ipair, bt, X, skip, pt),
+            (n, 2, 0, ipair, bt, P.tps_transform(2, 0, len(bt), X, L=3.0 * n)[0], skip, pt))
+
+
+@pytest.mark.parametrize("n,R,form,passes", [(19, 16, "complex", 2), (14, 16, "complete", 1), (21, 6, "complete", 2),
+                                             (17, 2, "diagonal", 1), (20, 8, "diagonal", 2)])
+def test_class_tiled_forms_match_the_oracle(n, R, form, passes):
+    """Complex couplings in two passes (beyond 2^22 elements W is read again and the sums span
+    the passes), members without a variant, and the complex-diagonal form: H.V and prdct as
+    the oracle's to 1e-12; mTPQ (four sums a step) to 1e-10, Hermitian forms."""
+    gm, om, shifted = _odd_model(n, form)
+    ctx = P.Context(gm, R=R)
+    got = gm.plan(R)
+    assert got["tile_states"] == 2048 // {2: 2, 6: 2, 8: 8, 16: 8}[R] and got["tile_passes"] == passes
+    rng = np.random.default_rng(n + R)
+    D = gm.dim
+    v1 = rng.standard_normal((D, R)) + 1j * rng.standard_normal((D, R))
+    v0 = 0.2 * rng.standard_normal((D, R)) + 0.1j * rng.standard_normal((D, R))
+    w = np.ascontiguousarray(v0).reshape(-1).copy()
+    pr = ctx.p_mltply_v3(np.ascontiguousarray(v1).reshape(-1), w, 0.0625)
+    w = w.reshape(D, R)
+    for r in sorted({0, 1, R // 2, R - 1}):
+        ref = np.ascontiguousarray(v0[:, r]).copy()
+        prr = om.p_mltply_v3(np.ascontiguousarray(v1[:, r]), ref, 0.0625)
+        assert rel(w[:, r], ref) <= 1e-12
+        assert abs(pr[r] - prr) <= 1e-12 * np.linalg.norm(v1[:, r]) * np.linalg.norm(ref)
+    ctx.close()
+    if form == "diagonal":
+        return
+    gt, ot = P.Model(*shifted), O.Model(*shifted)
+    V = np.ascontiguousarray(v1 / np.linalg.norm(v1, axis=0))
+    out = P.Context(gt, R=R).tps(3.0 * n, V.reshape(-1), 6)
+    for r in (0, R - 1):
+        ref = ot.tps(3.0 * n, np.ascontiguousarray(V[:, r]), 6)
+        assert rel(out["alpha"][:, r], ref["alpha"]) <= 1e-10 and rel(out["beta"][:, r], ref["beta"]) <= 1e-10
+        assert rel(out["coef"][:, r, :5], ref["coef"][:, :5]) <= 1e-10
+
+
+def test_class_tiled_single_vector_n26():
+    """One vector with complex couplings from 26 sites on: the default kernel's H.v on three
+    slices of 2^20 states against the oracle (1e-12), its <v|Hv> against a reduction of the
+    returned vector, and a short mTPQ and Lanczos run against the same run through the
+    gather kernel's plan (1e-10)."""
+    from pned_b200.lattice import cluster_for_sites
+    cl = cluster_for_sites(26)
+    gm, om = models(cl, 2, 0, KHGH, FIELD)
+    D, S = gm.dim, 1 << 20
+    ctx = P.Context(gm, R=1)
+    assert gm.plan(1) | {"partner_tiles": 0} == {"tile_passes": 2, "partner_tiles": 0, "tile_states": 2048,
+                                                 "staging": 0, "ring_stages": 0}
+    v1 = torch.empty(D, dtype=torch.complex128, device="cuda")
+    ctx.fill_gaussian(20261205, v1)
+    torch.cuda.synchronize()
+    host = v1.cpu().numpy()
+    w = torch.zeros_like(v1)
+    torch.cuda.synchronize()
+    pr = ctx.p_mltply_v3(v1, w, 0.0625)[0]
+    for lo in (0, D // 2 + 3 * S // 4, D - S):
+        ref = np.zeros(S, dtype=np.complex128)
+        om.p_mltply_v3_slice(host, ref, lo, lo + S, 0.0625)
+        assert rel(w[lo:lo + S].cpu().numpy(), ref) <= 1e-12
+    scale = float(torch.sum(torch.abs(v1) * torch.abs(w)).item())
+    assert abs(pr - complex(torch.vdot(v1, w).item())) <= 1e-12 * scale
+    runs = [(ctx.lanczos(v1, 6), ctx.tps(60.0, v1, 6))]
+    ctx.close()
+    assert gm.set_plan(1, 8, 10, 4, 3) != gm.set_plan(1)
+    gm.set_plan(1, 8, 10, 4, 3)
+    ctx = P.Context(gm, R=1)
+    runs.append((ctx.lanczos(v1, 6), ctx.tps(60.0, v1, 6)))
+    ctx.close()
+    for a, b in zip(*runs):
+        assert rel(a["alpha"], b["alpha"]) <= 1e-10 and rel(a["beta"], b["beta"]) <= 1e-10
+    del v1, w
+    torch.cuda.empty_cache()
+
+
+@pytest.mark.parametrize("form", ["real", "complex", "diagonal"])
+def test_s1_single_vector_forms_match_the_oracle(form):
+    """The nine-state S = 1 kernel at its smallest size, in each of its forms, with one sum
+    (H.v) and with four (mTPQ)."""
+    n = 9
+    ipair = np.array([[i + 1, i + 2] for i in range(n - 1)] + [[1, 5]], dtype=np.int32).reshape(-1)
+    bt = np.array([1 + i % 3 for i in range(n)], dtype=np.int32)
+    X, skip, pt = P.build_xlocal(3, 1, CP.kitaev_heisenberg(0.2, -1.0, gamma=0.0 if form == "real" else 0.1),
+                                 field=None if form == "real" else FIELD)
+    X = X.copy()
+    if form == "diagonal":
+        for t in range(9):
+            for i in range(9):
+                X[t, i, i] += 0.01j * (i + 1) * (t + 1)
+    args = (n, 3, 1, ipair, bt, X, skip, pt)
+    gm, om = P.Model(*args), O.Model(*args)
+    ctx = P.Context(gm, R=1)
+    assert gm.plan(1)["tile_states"] == 3 ** 7 and gm.plan(1)["tile_passes"] >= 1
+    rng = np.random.default_rng(3)
+    v1 = rng.standard_normal(gm.dim) + 1j * rng.standard_normal(gm.dim)
+    v0 = 0.2 * rng.standard_normal(gm.dim) + 0.1j * rng.standard_normal(gm.dim)
+    w, ref = v0.copy(), v0.copy()
+    pr, prr = ctx.p_mltply_v3(v1, w, 0.0625), om.p_mltply_v3(v1, ref, 0.0625)
+    assert rel(w, ref) <= 1e-12 and abs(pr[0] - prr) <= 1e-12 * np.linalg.norm(v1) * np.linalg.norm(ref)
+    if form == "diagonal":
+        return
+    L = 3.0 * n
+    args = args[:5] + (P.tps_transform(3, 1, len(bt), X, L=L)[0],) + args[6:]
+    v = v1 / np.linalg.norm(v1)
+    out, ref = P.Context(P.Model(*args), R=1).tps(L, v, 10), O.Model(*args).tps(L, v, 10)
+    assert rel(out["alpha"][:, 0], ref["alpha"]) <= 1e-10 and rel(out["beta"][:, 0], ref["beta"]) <= 1e-10
+    assert rel(out["coef"][:, 0, :5], ref["coef"][:, :5]) <= 1e-10

@@ -270,3 +270,62 @@ def test_slot_batches_take_the_class_tiled_kernel_where_it_is_the_faster(n, R, s
     sb = P.SlotBatch(P.ModelInput.structure(cluster_for_sites(n)), R, 4)
     assert sb.plan()["tile_states"] == states
     sb.close()
+
+
+@pytest.mark.parametrize("n,R,passes", [(18, 2, 1), (16, 12, 1), (22, 2, 2)])
+def test_slot_tables_in_the_class_tiled_kernel_match_the_oracle(n, R, passes):
+    """Slot batches large enough for the class-tiled kernel, each slot with its own couplings,
+    in one pass and in two: Lanczos and mTPQ slots as the oracle's runs."""
+    cl = cluster_for_sites(n)
+    steps, L = 8, 2.0 * n
+    sb = P.SlotBatch(P.ModelInput.structure(cl), R, steps)
+    got = sb.plan()
+    assert got["tile_states"] == 2048 // {2: 2, 12: 4}[R] and got["tile_passes"] == passes
+    runs = []
+    for r in range(R):
+        kind = "tps" if r % 2 else "lanczos"
+        cpl, fld = request_couplings(*REQS[r % 4])
+        slot_in, om = inputs(cl, cpl, fld, tps_L=L if kind == "tps" else None)
+        v = O.gaussian(200 + r, sb.dim)
+        v /= np.linalg.norm(v)
+        sb.load(r, kind, slot_in, v, steps, L=L)
+        runs.append((kind, om, v))
+    sb.step(steps)
+    for r in sorted({0, 1, R // 2, R - 1}):
+        kind, om, v = runs[r]
+        out = sb.read(r)
+        assert out["steps"] == steps and out["status"] == 0
+        ref = om.tps(L, v, steps) if kind == "tps" else om.lanczos(v, steps)
+        assert rel(out["alpha"], ref["alpha"]) <= 1e-10 and rel(out["beta"], ref["beta"]) <= 1e-10
+        if kind == "tps":
+            for j in range(5):
+                assert rel(out["coef"][:, j], ref["coef"][:, j]) <= 1e-10, j
+    sb.close()
+
+
+def test_one_slot_of_26_sites_matches_the_models_chain():
+    """A one-slot batch of 26 sites (the class-tiled kernel with a table that changes, four
+    sums a step) gives the Lanczos coefficients of a model with the same couplings, whose H.v
+    the parity tests compare with the oracle."""
+    cl = cluster_for_sites(26)
+    cpl, fld = request_couplings(*REQS[0])
+    steps = 6
+    v = torch.empty(1 << 26, dtype=torch.complex128, device="cuda")
+    P.api.gaussian_column(1 << 26, 1, 0, 5, v)
+    torch.cuda.synchronize()
+    v /= torch.linalg.vector_norm(v)
+    torch.cuda.synchronize()
+    m = P.Model.from_couplings(cl, cpl, field=fld)
+    ctx = P.Context(m, R=1)
+    ref = ctx.lanczos(v, steps)
+    ctx.close()
+    m.close()
+    sb = P.SlotBatch(P.ModelInput.structure(cl), 1, steps)
+    assert sb.plan()["tile_states"] == 2048 and sb.plan()["tile_passes"] == 2
+    sb.load(0, "lanczos", P.ModelInput.from_couplings(cl, cpl, field=fld), v, steps)
+    sb.step(steps)
+    out = sb.read(0)
+    assert rel(out["alpha"], ref["alpha"][:, 0]) <= 1e-10 and rel(out["beta"], ref["beta"][:, 0]) <= 1e-10
+    sb.close()
+    del v
+    torch.cuda.empty_cache()

@@ -355,7 +355,15 @@ def test_tuned_plans_are_kept_apart_by_coupling_type_and_candidate_set():
 
 
 XTILE_CASES = [(14, 16, True), (16, 4, False), (18, 2, True), (26, 1, True), (18, 4, True), (18, 6, False), (20, 8, True),
-               (28, 1, False), (24, 12, False), (24, 16, True)]
+               (28, 1, False), (24, 12, False), (24, 16, True), (14, 16, "complete"), (18, 4, "complete")]
+
+
+def _complete_graph(n, k):
+    """k sites all coupled to one another, the rest a chain: every three sites share neighbours,
+    so some members have no variant of their own."""
+    bonds = [(i, j) for i in range(k) for j in range(i + 1, k)] + [(i, i + 1) for i in range(k - 1, n - 1)]
+    return (np.array([[i + 1, j + 1] for i, j in bonds], dtype=np.int32).reshape(-1),
+            np.array([1 + i % 3 for i in range(len(bonds))], dtype=np.int32))
 
 
 @pytest.mark.parametrize("n,R,field", XTILE_CASES)
@@ -366,10 +374,16 @@ def test_class_tiled_plan_matches_every_flip_term(n, R, field):
     ones of the flip term itself (sampled states, the lowest and the highest
     included)."""
     from pned_b200.lattice import cluster_for_sites
-    cl = cluster_for_sites(n)
+    ipair, btype = _complete_graph(n, 9) if field == "complete" else (cluster_for_sites(n).ipair,
+                                                                      cluster_for_sites(n).ibond_type)
     cpl = CP.kitaev_heisenberg(0.6, 1.6, gamma=0.1 if field else 0.0)
     X, skip, pt = P.build_xlocal(2, 0, cpl, field=CP.field_111(0.05) if field else None)
-    r = api.xtile_plan_export(P.ModelInput(n, 2, 0, cl.ipair, cl.ibond_type, X, skip, pt), R)
+    r = api.xtile_plan_export(P.ModelInput(n, 2, 0, ipair, btype, X, skip, pt), R)
+    packs = [m["pack"] for ps in r["passes"] for m in ps["members"]]
+    # generic members where there are any; members marked real: all without a field, some with one
+    assert any(p & 15 == 14 for p in packs) or field != "complete"
+    real = [bool(p & (1 << 13)) for p in packs]
+    assert all(real) if not field else any(real) and not all(real)
     lr, D, M = r["lr"], [0, 0, 0, 0, 0, 0, 0, 0, 1, 2, 4, 3, 5, 6], [0, 1, 2, 4, 3, 5, 6, 7, 1, 2, 4, 3, 5, 6]
     assert R % (1 << lr) == 0
     dim = 1 << n
