@@ -122,7 +122,10 @@ template <bool RC, bool RD, int K, bool SLOT>
 __global__ void __launch_bounds__(kThreads, 2)
     hv_xtile_kernel(const __grid_constant__ XTileProgram prog, const HvArgs a, int nch)
 {
-    extern __shared__ double2 smem[];
+    // 128-byte aligned: a warp's rows then fill whole shared-memory lines.  Without it the static
+    // arrays in front decide (H.V with four sums, N = 22, R = 16 with a field: 3.55 ms 16 bytes off a
+    // line, 3.46 ms 32 bytes off, 3.42 ms aligned; N = 20, R = 6: 0.371, 0.350, 0.350)
+    extern __shared__ __align__(128) double2 smem[];
     const uint32_t tid = threadIdx.x;
     const int lr = prog.lr, rc = 1 << lr, R = a.R;
     const int ch = int(blockIdx.x) % nch;            // the block's group of vectors
