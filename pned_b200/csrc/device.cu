@@ -1084,13 +1084,16 @@ cudaError_t launch_hv_sums(const pned_model *m, const HvArgs &a, int nblocks, do
 {
     const int64_t rows = hv_partials(m, a, nblocks);
     const int kr = a.K * a.R;
-    const bool staged = a.R == 1 && !m->tprogs.empty() && m->use_tile && !find_xtiles(m, 1) && tile_staged(m);
     HvArgs b = a;
-    // the S = 1 kernel (its block size varies) and the sector's segment kernel (at its register
-    // limit: 1 % slower with the sums in it, N = 28) leave them to the finish kernels
-    const bool flat = !find_xtiles(m, a.R) && !(a.R == 1 && !m->tprogs.empty() && m->use_tile) && !find_qtiles(m, a.R);
-    const bool in = a.fin.done && kr == 1 && !staged && !find_q3(m, a.R) && !sector_segments_on(m) &&
-                    rows <= (flat ? std::min<int64_t>(kFinishInKernel, kFlatBlocksPerSM * m->nsm) : kFinishInKernel);
+    bool in = a.fin.done && kr == 1 && rows <= kFinishInKernel;
+    if (in) {
+        // the staged tile kernels, the S = 1 kernel (its block size varies) and the sector's
+        // segment kernel (at its register limit: 1 % slower with the sums in it, N = 28) leave
+        // them to the finish kernels
+        const bool xt = find_xtiles(m, 1) != nullptr, tile = !xt && !m->tprogs.empty() && m->use_tile;
+        in = !(tile && tile_staged(m)) && !(m->q == 3 && find_q3(m, 1)) && !sector_segments_on(m) &&
+             (rows <= kFlatBlocksPerSM * m->nsm || xt || tile || find_qtiles(m, 1));
+    }
     if (in) {
         b.fin.base = a.partials;
         b.fin.out = out;
