@@ -1027,14 +1027,14 @@ int plan_xtiles_for(const HostProgram &P, int R, int &lr, std::vector<XTilePass>
     if (R == 6 && double(P.dim) * R < double(1 << 19)) return PNED_ENOTSUP;
     // Tiles of 2048 elements: up to 8 vectors of 2^(11 - lr) states.  A warp's global read
     // moves 128 bytes a wavefront only from whole lines, so groups are as wide as R divides
-    // (8 vectors: 128-byte runs; N = 24, R = 16: 14.8 ms against 16.6 ms with groups of 4 and
-    // 25 ms with groups of 2), and narrower ones keep the low site bits in the tile (one
-    // vector: 4, N = 26: 3.74 ms against 3.85 with 3 and 3.78 with 5).
+    // (8 vectors: 128-byte runs; N = 24, R = 16: 12.6 ms against 14.7 ms with groups of 4 and
+    // 18.5 ms with groups of 2), and narrower ones keep the low site bits in the tile (one
+    // vector: 4, N = 26: 3.21 ms against 3.24 with 3 and 3.33 with 5).
     while (lr < 3 && R % (2 << lr) == 0) ++lr;
     const int fixed[4] = {4, 2, 1, 0};
-    // Up to 2^22 elements (64 MB) the vectors stay in L2: one pass (N = 18, R = 16: 0.22 ms
-    // against 0.26 ms).  Beyond, two: their tiles hold most masks, so fewer partner tiles
-    // come from memory (N = 26, R = 4: 14.3 ms against 22.3 ms with one and 15.1 ms with three).
+    // Up to 2^22 elements (64 MB) the vectors stay in L2: one pass (N = 18, R = 16: 0.227 ms
+    // against 0.254 ms).  Beyond, two: their tiles hold most masks, so fewer partner tiles
+    // come from memory (N = 26, R = 4: 13.0 ms against 21.9 ms with one and 13.4 ms with three).
     const int passes = double(P.dim) * R <= double(1 << 22) ? 1 : 2;
     return plan_xtiles(P, 11 - lr, fixed[lr], passes, out);
 }

@@ -43,9 +43,9 @@ __device__ __forceinline__ void q3_apply(const double2 *ct, const double2 (&w)[k
 // state; the kernel for any base (hv_qtile.cu) reads a coefficient and decodes the pair
 // state for every state and term as well.
 //
-// What bounds it: instructions and shared-memory reads, not memory (N = 16: 3.7 ms for 5
-// passes that move 10 GB).  H.v of one vector: N = 18 50.2 -> 32 ms, N = 16 5.52 -> 3.68 ms,
-// N = 14 with a field 1.15 -> 0.64 ms, N = 12 0.120 -> 0.089 ms.  Rows and the epilogue's
+// What bounds it: instructions and shared-memory reads, not memory (N = 16: 3.66 ms for 5
+// passes that move 10 GB).  H.v of one vector: N = 18 50.2 -> 32.3 ms, N = 16 5.57 -> 3.66 ms,
+// N = 14 with a field 1.20 -> 0.66 ms; Lanczos step N = 12 0.113 -> 0.080 ms.  Rows and the epilogue's
 // P or W and diagonal come in by cp.async in global order; local slots are nine apart from
 // lane to lane, so the 16-byte reads have no bank conflicts.
 template <bool RC, bool RD, int K>
@@ -266,8 +266,9 @@ cudaError_t launch_q3(const pned_model *m, const pned_model::Q3Set &qs, const Hv
 }
 
 // The S = 1 passes for one vector (several: the kernel for any base runs, whose threads
-// share a term's decode over their vectors; N = 16, R = 4: 20.6 against 21.6 ms a step,
-// N = 12, R = 8: 0.41 against 0.52 ms): the largest tile whose two buffers, tables and index
+// share a term's decode over their vectors; a form of this kernel with all vectors in one
+// tile took 21.6 against 20.6 ms a step at N = 16, R = 4, and 0.52 against 0.41 ms at N = 12,
+// R = 8): the largest tile whose two buffers, tables and index
 // arrays leave room for two blocks per SM.  From 9 sites on: at 8 a tile is 729 states, 81
 // items, so nine blocks of three warps run, each thread's nine states one after another
 // (Lanczos step 31.1 against 27.2 us with the kernel for any base, mTPQ step 35.9 against

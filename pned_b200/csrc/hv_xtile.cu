@@ -109,15 +109,16 @@ __device__ __forceinline__ void x_member(const uint4 &S, uint32_t base, uint32_t
 // own rows come into shared memory by cp.async and the in-tile classes gather there;
 // the out-of-tile classes read their partner rows through L1/L2 meanwhile.
 //
-// What bounds it: not memory (N = 22, R = 16 with a field: DRAM at a quarter of its
-// rate, the L1 data path 50 % busy) but instructions and their latency at 16 warps per
-// SM: fp64 pipe 28 %, issue 46 %.  Hence the classes (60 masks become 40 row reads at
+// What bounds it: not memory (N = 22, R = 16 with a field: DRAM at a third of its
+// rate, the L1 data path 50-58 % busy) but instructions and their latency at 16 warps per
+// SM: fp64 pipe 25 %, issue 48 %.  Hence the classes (60 masks become 40 row reads at
 // N = 24), the perfect hash (3 instructions for a coefficient index), members as one
 // 16-byte constant read fetched ahead, and the indexed jump.  Measured H.V against the
-// multi-vector kernel: N = 24, R = 16 with a field 18.6 -> 13.0 ms, R = 12 without
-// 12.0 -> 8.3 ms, N = 22, R = 2 0.69 -> 0.49 ms, N = 26, R = 4 21.5 -> 14.3 ms.
-// Measured and dropped: a second class in flight through cp.async (15.1 against 14.8 ms:
-// the address arithmetic costs more than the latency it hides).
+// multi-vector kernel: N = 24, R = 16 with a field 18.6 -> 12.6 ms, R = 12 without
+// 11.8 -> 8.1 ms, N = 22, R = 2 with a field 0.675 -> 0.429 ms, N = 26, R = 4 with a field
+// 21.5 -> 13.0 ms, without 14.9 -> 9.5 ms.
+// Measured and dropped, on an earlier form: a second class in flight through cp.async (15.1
+// against 14.8 ms: the address arithmetic costs more than the latency it hides).
 template <bool RC, bool RD, int K, bool SLOT>
 __global__ void __launch_bounds__(kThreads, 2)
     hv_xtile_kernel(const __grid_constant__ XTileProgram prog, const HvArgs a, int nch)
@@ -324,8 +325,8 @@ bool ensure_xtiles(pned_model *m, int R, bool slot_tables)
     if (pick_vpt(R) == 0) return false;
     // One vector: only for complex coefficients (Gamma, a field, slot couplings) -- with real
     // ones a member is half the products, and the tensor-copy kernel is faster -- and only from
-    // 26 sites on (N = 26: 4.20 -> 3.63 ms, N = 28: 16.0 -> 15.1 ms).  Smaller bases keep the
-    // gather kernel's order of additions although it is slower (N = 24: 1.04 against 0.93 ms):
+    // 26 sites on (N = 26: 3.88 -> 3.21 ms, N = 28: 16.1 -> 14.0 ms).  Smaller bases keep the
+    // gather kernel's order of additions although it is slower (N = 24: 0.98 against 0.82 ms):
     // the sign of the Ritz vector that vec12 finds turns on the last bit of alpha and beta, so
     // another order may return -x where a caller had x.
     if (R == 1 && (m->real_coef || hp.n < kTileBigSites)) return false;
